@@ -1,6 +1,7 @@
 // Field preparation kernels: raw 8-variable frames -> 32-variable arrays
 // with gradients (mhd_data_parallel.f90:504-610) -> packed mover records.
 #include "device_common.cuh"
+#include "fp64_exact.cuh"
 
 namespace gpat {
 
@@ -155,8 +156,9 @@ cudaError_t launch_fill(float *a, float v, size_t n, cudaStream_t s) {
 
 template <int R>
 __global__ void pack_kernel(const float *__restrict__ full, float *__restrict__ rec,
-                            size_t ncells) {
+                            size_t ncells, unsigned int *odd_found) {
     const size_t stride = (size_t)gridDim.x * blockDim.x;
+    bool odd = false;
     for (size_t c = (size_t)blockIdx.x * blockDim.x + threadIdx.x; c < ncells; c += stride) {
         const float *src = full + 32 * c;
         float *dst = rec + (size_t)R * c;
@@ -165,16 +167,38 @@ __global__ void pack_kernel(const float *__restrict__ full, float *__restrict__ 
             const int v = (R == kRec2D) ? kPack2D[r] : kPack3D[r];
             dst[r] = v >= 0 ? src[v] : 0.0f;
         }
+#pragma unroll
+        for (int v = 0; v < 32; ++v) odd |= odd_float(src[v]);
     }
+    if (odd) *odd_found = 1u;
+}
+
+__global__ void find_odd_kernel(const float *__restrict__ a, size_t n, unsigned int *odd_found) {
+    const size_t stride = (size_t)gridDim.x * blockDim.x;
+    bool odd = false;
+    for (size_t c = (size_t)blockIdx.x * blockDim.x + threadIdx.x; c < n; c += stride)
+        odd |= odd_float(a[c]);
+    if (odd) *odd_found = 1u;
+}
+
+cudaError_t launch_find_odd(const float *a, size_t n, unsigned int *odd, cudaStream_t s) {
+    const cudaError_t e = cudaMemsetAsync(odd, 0, sizeof(unsigned int), s);
+    if (e != cudaSuccess || n == 0) return e;
+    const size_t blocks = (n + 255) / 256;
+    find_odd_kernel<<<(unsigned)(blocks < 65535 ? blocks : 65535), 256, 0, s>>>(a, n, odd);
+    return cudaGetLastError();
 }
 
 cudaError_t launch_pack_records(const float *full, float *rec, int ndim, size_t ncells,
-                                cudaStream_t s) {
+                                unsigned int *odd, cudaStream_t s) {
+    const cudaError_t e = cudaMemsetAsync(odd, 0, sizeof(unsigned int), s);
+    if (e != cudaSuccess) return e;
     const int threads = 256;
     size_t blocks = (ncells + threads - 1) / threads;
     if (blocks > 65535 * 16) blocks = 65535 * 16;
-    if (ndim == 2) pack_kernel<kRec2D><<<(unsigned)blocks, threads, 0, s>>>(full, rec, ncells);
-    else pack_kernel<kRec3D><<<(unsigned)blocks, threads, 0, s>>>(full, rec, ncells);
+    if (ndim == 2) pack_kernel<kRec2D><<<(unsigned)blocks, threads, 0, s>>>(full, rec, ncells,
+                                                                           odd);
+    else pack_kernel<kRec3D><<<(unsigned)blocks, threads, 0, s>>>(full, rec, ncells, odd);
     return cudaGetLastError();
 }
 

@@ -10,6 +10,7 @@
 #include <new>
 #include <vector>
 
+#include "fp64_exact.cuh"
 #include "gpat_internal.h"
 
 using namespace gpat;
@@ -68,6 +69,9 @@ struct gpat_handle {
     // and the bins of that binning
     uint8_t *pause = nullptr;
     int64_t pause_cap = 0;
+    // FP64 mover: the order its lanes take the particles in
+    uint32_t *work = nullptr;
+    int64_t work_cap = 0;
     // learned splitting inside the mover (gpat_set_mover_learned): the
     // launch arguments, and on the device the particle count with children,
     // the judged count and the fixed-point sum of w exp(z - z_shift)
@@ -359,6 +363,15 @@ int mover_args(gpat_handle_t *h, int mhd_tframe, int nsteps_interval, int num_fi
     a.key1 = (uint32_t)(p.seed >> 32);
     a.trk = track_args(h);
     a.cnt = h->dcnt;
+    a.rdx = reciprocal(a.dx); a.rdy = reciprocal(a.dy); a.rdz = reciprocal(a.dz);
+    a.rdtf = reciprocal(a.dtf);
+    a.rp0 = reciprocal(a.p0);
+    a.d1p0 = a.drift1 * a.p0;
+    a.d2p0sq = a.drift2 * (a.p0 * a.p0);
+    auto usual = [](double v) { return std::fabs(v) > 1e-60 && std::fabs(v) < 1e60; };
+    a.drift_finite = a.charge != 0 && usual(a.d1p0) && usual(a.d2p0sq);
+    a.sdt_min = std::sqrt(a.dt_min);
+    a.sdt_max = std::sqrt(a.dt_max);
     a.pause = nullptr;
     return GPAT_OK;
 }
@@ -736,6 +749,7 @@ int gpat_destroy(gpat_handle_t *h) {
     if (h->sort_scratch) cudaFree(h->sort_scratch);
     if (h->tile_dev) cudaFree(h->tile_dev);
     if (h->pause) cudaFree(h->pause);
+    if (h->work) cudaFree(h->work);
     if (h->learn_dev) cudaFree(h->learn_dev);
     if (h->fresh_dev) cudaFree(h->fresh_dev);
     if (h->tile_ovf) cudaFree(h->tile_ovf);
@@ -801,7 +815,8 @@ int gpat_set_fields(gpat_handle_t *h, int var_flag, const float *farray, int nva
     if (nvar == 32) {
         CK(cudaMemcpyAsync(h->full[slot], farray, 32 * sizeof(float) * h->ncells,
                            cudaMemcpyHostToDevice, h->stream));
-        CK(launch_pack_records(h->full[slot], h->rec[slot], h->prm.ndim, h->ncells, h->stream));
+        CK(launch_pack_records(h->full[slot], h->rec[slot], h->prm.ndim, h->ncells,
+                               &h->dcnt->odd_fields[slot], h->stream));
         h->rec_ready[slot] = true;
         ++h->rec_gen[slot];
     } else {
@@ -836,6 +851,7 @@ int gpat_set_fluctuations(gpat_handle_t *h, int var_flag, const float *db2_slab,
     const gpat_mhd_config_t &c = h->cfg;
     CK(launch_calc_aux_gradients(h->aux[slot], h->prm.ndim, h->nxg, h->nyg, h->nzg, c.dx, c.dy,
                                  c.dz, h->stream, grad_spans(h)));
+    CK(launch_find_odd(h->aux[slot], 16 * h->ncells, &h->dcnt->odd_aux[slot], h->stream));
     CK(cudaStreamSynchronize(h->stream));
     return GPAT_OK;
 }
@@ -1028,7 +1044,8 @@ int gpat_calc_fields_gradients(gpat_handle_t *h, int var_flag) {
     const gpat_mhd_config_t &c = h->cfg;
     CK(launch_calc_fields_gradients(h->full[slot], h->prm.ndim, h->nxg, h->nyg, h->nzg, c.dx, c.dy,
                                     c.dz, h->stream, grad_spans(h)));
-    CK(launch_pack_records(h->full[slot], h->rec[slot], h->prm.ndim, h->ncells, h->stream));
+    CK(launch_pack_records(h->full[slot], h->rec[slot], h->prm.ndim, h->ncells,
+                           &h->dcnt->odd_fields[slot], h->stream));
     CK(cudaStreamSynchronize(h->stream));
     h->rec_ready[slot] = true;
     ++h->rec_gen[slot];
@@ -1043,6 +1060,10 @@ int gpat_copy_fields(gpat_handle_t *h) {
     CK(cudaMemcpyAsync(h->full[0], h->full[1], 32 * sizeof(float) * h->ncells,
                        cudaMemcpyDeviceToDevice, h->stream));
     CK(cudaMemcpyAsync(h->rec[0], h->rec[1], (size_t)R * sizeof(float) * h->ncells,
+                       cudaMemcpyDeviceToDevice, h->stream));
+    CK(cudaMemcpyAsync(&h->dcnt->odd_fields[0], &h->dcnt->odd_fields[1], sizeof(unsigned int),
+                       cudaMemcpyDeviceToDevice, h->stream));
+    CK(cudaMemcpyAsync(&h->dcnt->odd_aux[0], &h->dcnt->odd_aux[1], sizeof(unsigned int),
                        cudaMemcpyDeviceToDevice, h->stream));
     if (h->aux[0] && h->aux[1])   // copy_magnetic_fluctuation / copy_correlation_length
         CK(cudaMemcpyAsync(h->aux[0], h->aux[1], 16 * sizeof(float) * h->ncells,
@@ -1568,6 +1589,21 @@ int gpat_particle_mover(gpat_handle_t *h, int focused_transport, int nlgc, doubl
             h->nptl_split += h->learn_split;
         }
     } else {
+        if (mover_fp64_orders(h->n, h->sm_count)) {
+            if (h->n > h->work_cap) {
+                CK(cudaStreamSynchronize(h->stream));
+                if (h->work) CK(cudaFree(h->work));
+                h->work = nullptr;
+                h->work_cap = 0;
+                if (cudaMalloc(&h->work, sizeof(uint32_t) * ((size_t)h->cap + kOrderHead)) !=
+                    cudaSuccess) {
+                    cudaGetLastError();
+                    return fail(h, GPAT_ERR_OOM, "work list");
+                }
+                h->work_cap = h->cap;
+            }
+            a.work = h->work;
+        }
         CK(cudaEventRecord(h->ev0, h->stream));
         CK(launch_mover_fp64(a, h->sm_count, h->stream));
         CK(cudaEventRecord(h->ev1, h->stream));

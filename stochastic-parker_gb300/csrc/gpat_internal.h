@@ -50,6 +50,10 @@ struct DevCounters {
     unsigned long long bad_value;
     unsigned long long trk_dropped;  // tracked records past nsteps_tracking_max
     unsigned long long pmax_bits;    // get_pmax_global: bits of the largest p >= 0
+    unsigned long long next;         // FP64 mover launch: particles handed out so far
+    // per frame slot: some field value (or fluctuation value) is subnormal,
+    // infinite or NaN
+    unsigned int odd_fields[2], odd_aux[2];
 };
 
 // Packed per-cell field records read by the movers.  2D: 16 floats,
@@ -118,6 +122,15 @@ struct MoverArgs {
     const double *surf[2][2];   // [surface][frame]
     TrackArgs trk;              // FP64 mover only
     DevCounters *cnt;
+    // FP64 mover: rounded reciprocals of dx, dy, dz, dtf and p0 (div_by), and
+    // the products and roots of the run's constants that every push needs.
+    double rdx, rdy, rdz, rdtf, rp0, d1p0, d2p0sq, sdt_min, sdt_max;
+    int drift_finite;   // the drift's prefactor is finite for any momentum
+    // FP64 mover's work list: lanes of a warp that take particles, and the
+    // order they are taken in (kOrderHead words of scratch, then the indices;
+    // null: by index).
+    int lanes;
+    uint32_t *work;
 };
 
 // Single-precision constants of the split-precision mover, derived on the
@@ -212,8 +225,12 @@ cudaError_t launch_scatter_raw_fields(const float *raw, int nvar, float *full, s
 cudaError_t launch_calc_fields_gradients(float *full, int ndim, int nxg, int nyg, int nzg,
                                          double dx, double dy, double dz, cudaStream_t s,
                                          const double *const *ih = nullptr);
+// *odd (zeroed here) is set to 1 when one of the 32 variables of some cell is
+// subnormal, infinite or NaN (fp64_exact.cuh).
 cudaError_t launch_pack_records(const float *full, float *rec, int ndim, size_t ncells,
-                                cudaStream_t s);
+                                unsigned int *odd, cudaStream_t s);
+// The same over n floats.
+cudaError_t launch_find_odd(const float *a, size_t n, unsigned int *odd, cudaStream_t s);
 // Chunk-planar copy of packed records (R / 4 planes of float4, one per
 // 16-byte chunk of the record) for the tile mover.
 cudaError_t launch_planarize_records(const float *rec, float *planes, int ndim, size_t ncells,
@@ -227,6 +244,10 @@ cudaError_t launch_scatter_aux(const float *src, float *aux, int comp, size_t nc
                                cudaStream_t s);
 cudaError_t launch_fill(float *a, float v, size_t n, cudaStream_t s);
 cudaError_t launch_mover_fp64(const MoverArgs &a, int sm_count, cudaStream_t s);
+// Whether that launch orders n particles, for which MoverArgs::work has room
+// for kOrderHead + n words.
+constexpr int kOrderHead = 128;
+bool mover_fp64_orders(int64_t n, int sm_count);
 cudaError_t launch_mover_mixed(const MoverArgs &a, const MixedConsts &c, int sm_count,
                                cudaStream_t s);
 MixedConsts make_mixed_consts(const MoverArgs &a);
