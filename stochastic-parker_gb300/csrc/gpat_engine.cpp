@@ -539,6 +539,16 @@ int collect_escaped(gpat_handle_t *h) {
     return GPAT_OK;
 }
 
+// Host frames pass through a staging buffer of at most this many cells of 8
+// floats (128 MiB), a part at a time.
+constexpr size_t kStagingCells = (size_t)1 << 22;
+
+int ensure_staging(gpat_handle_t *h) {
+    if (h->staging) return GPAT_OK;
+    CK(cudaMalloc(&h->staging, 8 * sizeof(float) * std::min(kStagingCells, h->ncells)));
+    return GPAT_OK;
+}
+
 int ensure_scratch(gpat_handle_t *h, int64_t n) {
     const size_t need = compaction_scratch_bytes(n);
     if (need <= h->scratch_bytes) return GPAT_OK;
@@ -820,10 +830,14 @@ int gpat_set_fields(gpat_handle_t *h, int var_flag, const float *farray, int nva
         h->rec_ready[slot] = true;
         ++h->rec_gen[slot];
     } else {
-        if (!h->staging) CK(cudaMalloc(&h->staging, 8 * sizeof(float) * h->ncells));
-        CK(cudaMemcpyAsync(h->staging, farray, 8 * sizeof(float) * h->ncells,
-                           cudaMemcpyHostToDevice, h->stream));
-        CK(launch_scatter_raw_fields(h->staging, 8, h->full[slot], h->ncells, h->stream));
+        const int rc = ensure_staging(h);
+        if (rc) return rc;
+        for (size_t c = 0; c < h->ncells; c += kStagingCells) {
+            const size_t m = std::min(kStagingCells, h->ncells - c);
+            CK(cudaMemcpyAsync(h->staging, farray + 8 * c, 8 * sizeof(float) * m,
+                               cudaMemcpyHostToDevice, h->stream));
+            CK(launch_scatter_raw_fields(h->staging, h->full[slot] + 32 * c, m, h->stream));
+        }
         h->rec_ready[slot] = false;
     }
     CK(cudaStreamSynchronize(h->stream));
@@ -839,13 +853,17 @@ int gpat_set_fluctuations(gpat_handle_t *h, int var_flag, const float *db2_slab,
     if (!h->aux[slot])
         return fail(h, GPAT_ERR_STATE, "fluctuation arrays need deltab_flag or correlation_flag");
     CK(cudaSetDevice(h->device));
-    if (!h->staging) CK(cudaMalloc(&h->staging, 8 * sizeof(float) * h->ncells));
+    const int rcs = ensure_staging(h);
+    if (rcs) return rcs;
     const float *src[4] = {db2_slab, db2_2d, lc_slab, lc_2d};
     for (int g = 0; g < 4; ++g) {
         if (!src[g]) continue;
-        CK(cudaMemcpyAsync(h->staging, src[g], sizeof(float) * h->ncells, cudaMemcpyHostToDevice,
-                           h->stream));
-        CK(launch_scatter_aux(h->staging, h->aux[slot], 4 * g, h->ncells, h->stream));
+        for (size_t c = 0; c < h->ncells; c += 8 * kStagingCells) {
+            const size_t m = std::min(8 * kStagingCells, h->ncells - c);
+            CK(cudaMemcpyAsync(h->staging, src[g] + c, sizeof(float) * m, cudaMemcpyHostToDevice,
+                               h->stream));
+            CK(launch_scatter_aux(h->staging, h->aux[slot] + 16 * c, 4 * g, m, h->stream));
+        }
         CK(cudaStreamSynchronize(h->stream));   // staging is reused
     }
     const gpat_mhd_config_t &c = h->cfg;
@@ -1042,10 +1060,9 @@ int gpat_calc_fields_gradients(gpat_handle_t *h, int var_flag) {
     if (slot >= h->nslots || !h->fields_set[slot]) return fail(h, GPAT_ERR_STATE, "fields not set");
     CK(cudaSetDevice(h->device));
     const gpat_mhd_config_t &c = h->cfg;
-    CK(launch_calc_fields_gradients(h->full[slot], h->prm.ndim, h->nxg, h->nyg, h->nzg, c.dx, c.dy,
-                                    c.dz, h->stream, grad_spans(h)));
-    CK(launch_pack_records(h->full[slot], h->rec[slot], h->prm.ndim, h->ncells,
-                           &h->dcnt->odd_fields[slot], h->stream));
+    CK(launch_calc_fields_gradients(h->full[slot], h->rec[slot], h->prm.ndim, h->nxg, h->nyg, h->nzg,
+                                    c.dx, c.dy, c.dz, grad_spans(h), &h->dcnt->odd_fields[slot],
+                                    h->stream));
     CK(cudaStreamSynchronize(h->stream));
     h->rec_ready[slot] = true;
     ++h->rec_gen[slot];
@@ -1488,7 +1505,7 @@ int gpat_particle_mover(gpat_handle_t *h, int focused_transport, int nlgc, doubl
         s.item_counter = reinterpret_cast<unsigned long long *>(h->tile_dev + s.nbricks + 1);
         s.nodes = (uint32_t)((sx + 1) * (sy + 1) * (h->prm.ndim == 3 ? sz + 1 : 1));
         // chunk-planar copies of the frames' records, rebuilt when the records changed
-        const int R = (h->prm.ndim == 2) ? kRec2D : kRec3D;
+        const int R = 4 * ((h->prm.ndim == 2) ? kChunks2D : kChunks3D);
         for (int slot = 0; slot < (a.time_interp ? 2 : 1); ++slot) {
             if (!h->planes[slot]) {
                 if (cudaMalloc(&h->planes[slot], (size_t)R * sizeof(float) * h->ncells) !=
@@ -2256,7 +2273,7 @@ int gpat_batch_create(gpat_handle_t *const *runs, int nruns, gpat_batch_t **out)
     b->ndim = h0->prm.ndim;
     int variants[4];
     batch_minb_variants(b->ndim, variants);
-    b->tuning.minb = b->ndim == 2 ? 6 : 5;   // the single-run kernel's register target
+    b->tuning.minb = b->ndim == 2 ? 6 : 4;   // the single-run kernel's register target
     b->tuning.grab = 1;
     cudaSetDevice(b->device);
     if (cudaStreamCreateWithFlags(&b->stream, cudaStreamNonBlocking) != cudaSuccess ||
@@ -2354,7 +2371,7 @@ int gpat_batch_autotune(gpat_batch_t *b, const int *mhd_tframe, int nlgc, double
     const int chunks[3] = {64, 128, 256};
     gpat_batch_tuning_t top{};
     top.pushes_per_s = -1.0;
-    const int def_minb = b->ndim == 2 ? 6 : 5;
+    const int def_minb = b->ndim == 2 ? 6 : 4;
     const int bi0 = b->runs[0]->prm.bin_interval;
     const int def_chunk = bi0 == 0 ? 128 : (bi0 > 0 ? bi0 : 0);
     double def_rate = 0.0;

@@ -56,10 +56,15 @@ struct DevCounters {
     unsigned int odd_fields[2], odd_aux[2];
 };
 
-// Packed per-cell field records read by the movers.  2D: 16 floats,
-// 3D: 24 floats (see fields.cu for the slot order).
+// Packed per-cell field records read by the movers (see fields.cu for the slot
+// order).  2D: 16 floats; 3D: 24 floats, the first 21 of them read, in a
+// 128-byte line of their own: a group of lanes then reads a record's sectors
+// with one tag lookup (2.0e11 random records/s against 1.4e11 at a stride of
+// 96 bytes, where half of the records span two lines).  The brick mover's
+// chunk planes hold the 24 floats.
 constexpr int kRec2D = 16;
-constexpr int kRec3D = 24;
+constexpr int kRec3D = 32;
+constexpr int kChunks2D = 4, kChunks3D = 6;   // 16-byte chunks with data
 
 // Particle tracking (track_particle_flag, particle_module.f90:144-150):
 // tags_tracking(nrows, n) and particles_tracked(nsteps_max, n), both in
@@ -218,21 +223,24 @@ struct MlpTrainBuffers {
 };
 
 // Launchers (defined in the .cu files).  All enqueue on `s`.
-cudaError_t launch_scatter_raw_fields(const float *raw, int nvar, float *full, size_t ncells,
+// raw: 8 variables per cell; the gradients of full become 0.
+cudaError_t launch_scatter_raw_fields(const float *raw, float *full, size_t ncells,
                                       cudaStream_t s);
-// ih: per-axis inverse spans of a non-uniform grid (3 device pointers), or
-// null for the uniform 0.5 / d.
-cudaError_t launch_calc_fields_gradients(float *full, int ndim, int nxg, int nyg, int nzg,
-                                         double dx, double dy, double dz, cudaStream_t s,
-                                         const double *const *ih = nullptr);
-// *odd (zeroed here) is set to 1 when one of the 32 variables of some cell is
-// subnormal, infinite or NaN (fp64_exact.cuh).
+// Gradients into full and the packed records in one pass.  ih: per-axis inverse
+// spans of a non-uniform grid (3 device pointers), or null for the uniform
+// 0.5 / d.  *odd (zeroed here) is set to 1 when one of the 32 variables of some
+// cell is subnormal, infinite or NaN (fp64_exact.cuh).
+cudaError_t launch_calc_fields_gradients(float *full, float *rec, int ndim, int nxg, int nyg,
+                                         int nzg, double dx, double dy, double dz,
+                                         const double *const *ih, unsigned int *odd,
+                                         cudaStream_t s);
+// The packed records alone (frames that come with their gradients); odd as above.
 cudaError_t launch_pack_records(const float *full, float *rec, int ndim, size_t ncells,
                                 unsigned int *odd, cudaStream_t s);
 // The same over n floats.
 cudaError_t launch_find_odd(const float *a, size_t n, unsigned int *odd, cudaStream_t s);
-// Chunk-planar copy of packed records (R / 4 planes of float4, one per
-// 16-byte chunk of the record) for the tile mover.
+// Chunk-planar copy of packed records (planes of float4, one per 16-byte chunk
+// of the record that holds data) for the tile mover.
 cudaError_t launch_planarize_records(const float *rec, float *planes, int ndim, size_t ncells,
                                      cudaStream_t s);
 // Fluctuation records: 16 floats per node, {db2_slab, db2_2d, lc_slab,

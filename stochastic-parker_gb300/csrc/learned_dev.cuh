@@ -47,9 +47,10 @@ __device__ void particle_features(const FeatureArgs &g, const DevParticles &P, i
     const int iz = (NDIM == 3) ? min(max(cz + 2, 0), g.nzg - 2) : 0;
     fx = fminf(fmaxf(fx, 0.0f), 1.0f); fy = fminf(fmaxf(fy, 0.0f), 1.0f);
     fz = fminf(fmaxf(fz, 0.0f), 1.0f);
-    float v[R];
+    constexpr int NV = (NDIM == 2) ? 15 : 21;
+    float v[NV];
 #pragma unroll
-    for (int k = 0; k < R; ++k) v[k] = 0.0f;
+    for (int k = 0; k < NV; ++k) v[k] = 0.0f;
     for (int kk = 0; kk < (NDIM == 3 ? 2 : 1); ++kk)
         for (int j = 0; j < 2; ++j)
             for (int ii = 0; ii < 2; ++ii) {
@@ -59,7 +60,7 @@ __device__ void particle_features(const FeatureArgs &g, const DevParticles &P, i
                                     (size_t)g.nxg * ((size_t)(iy + j) + (size_t)g.nyg * (iz + kk));
                 const float *r = g.rec + (size_t)R * cell;
 #pragma unroll
-                for (int k = 0; k < R; ++k) v[k] = fmaf(__ldg(r + k), w, v[k]);
+                for (int k = 0; k < NV; ++k) v[k] = fmaf(__ldg(r + k), w, v[k]);
             }
     f[0] = (float)((P.x[i] - g.xmin) * g.ilx);
     f[1] = (float)((P.y[i] - g.ymin) * g.ily);

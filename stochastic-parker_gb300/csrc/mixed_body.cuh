@@ -225,7 +225,7 @@ struct TileGather {
     template <int NDIM, int NV>
     __device__ __forceinline__ bool interp(const MixedRunArgs &a, const Pos &q, float rt,
                                            float f[NV]) const {
-        constexpr int R4 = ((NDIM == 2) ? kRec2D : kRec3D) / 4;
+        constexpr int R4 = (NDIM == 2) ? kChunks2D : kChunks3D;
         const int ix = q.cx + 2, iy = q.cy + 2, iz = (NDIM == 3) ? q.cz + 2 : 0;
         if ((unsigned)ix > (unsigned)(a.nxg - 2) || (unsigned)iy > (unsigned)(a.nyg - 2) ||
             (NDIM == 3 && (unsigned)iz > (unsigned)(a.nzg - 2))) {
