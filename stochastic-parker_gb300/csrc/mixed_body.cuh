@@ -77,14 +77,16 @@ __device__ __forceinline__ void negp_or_boundary(const MixedRunArgs &a, const Mi
     if (p < 0.0f) {
         flag = 0;
         atomic_add_fixed(&a.cnt->negp_hi, &a.cnt->negp_lo, *w);
-    } else {
+    } else if ((unsigned)q.cx >= (unsigned)k.nx || (unsigned)q.cy >= (unsigned)k.ny ||
+               (NDIM == 3 && (unsigned)q.cz >= (unsigned)k.nz)) {
+        // not in one of the box's own cells
         boundary<NDIM>(a, k, q, true, flag, w);
     }
 }
 
 // 256-bit read-only global load (8 floats, 32-byte aligned address).  Records
-// are 64 B (2D) or 96 B (3D) at 32-byte aligned offsets, so one corner costs 2
-// or 3 of these instead of 4 or 6 128-bit loads.
+// are 64 B (2D) or 96 B in a 128-byte line (3D), so one corner costs 2 or 3 of
+// these instead of 4 or 6 128-bit loads.
 __device__ __forceinline__ void ld8(const float *p, float (&v)[8]) {
     asm("ld.global.nc.v8.f32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
         : "=f"(v[0]), "=f"(v[1]), "=f"(v[2]), "=f"(v[3]), "=f"(v[4]), "=f"(v[5]), "=f"(v[6]),
@@ -153,6 +155,108 @@ __device__ __forceinline__ bool interp_global(const MixedRunArgs &a, const Pos &
                 }
             }
     return true;
+}
+
+// interp_global for a whole warp, each lane's particle by a group of lanes:
+// lane j of a group of 2 (2D) or 4 (3D) reads the 32-byte sector j of a
+// corner's record for every particle of the group in turn, weighs and sums it,
+// and the sums change hands in shared memory.  A load instruction then touches
+// 16 (8) lines instead of 32 scattered sectors, and the L1 data pipe, which
+// spends a wavefront per line touched, delivers twice the records (random
+// records of 64 B: 2.3e11/s against 1.15e11; of 96 B: 1.96e11 against 9.9e10).
+// Weights and the order of the sums are interp_global's.  want: the lane's
+// particle makes a push.  All lanes of the warp call; buf: its kGatherBuf<NDIM>
+// floats.  False where the position is outside the ghost range.
+// The buffer holds planes of one 16-byte chunk per lane: plane j + sectors h is
+// half h of sector j, rotated by j lanes, so that neither the writes of a
+// group's sectors nor the reads of a plane share banks.  In 3D the last plane
+// keeps one float per lane, the 21st value.
+constexpr int kGatherPlane = 4 * 32;
+template <int NDIM>
+constexpr int kGatherBuf = NDIM == 2 ? 4 * kGatherPlane : 5 * kGatherPlane + 32;
+
+template <int NDIM, int NV>
+__device__ __forceinline__ bool interp_group(const MixedRunArgs &a, const Pos &q, float rt,
+                                             bool want, float *buf, float f[NV]) {
+    constexpr int R = (NDIM == 2) ? kRec2D : kRec3D;
+    constexpr int G = (NDIM == 2) ? 2 : 4, kSectors = (NDIM == 2) ? 2 : 3;
+    constexpr int kCorners = (NDIM == 2) ? 4 : 8;
+    const int lane = threadIdx.x & 31, sub = lane & (G - 1);
+    const int ix = q.cx + 2, iy = q.cy + 2, iz = (NDIM == 3) ? q.cz + 2 : 0;
+    bool ok = want;
+    if (want && ((unsigned)ix > (unsigned)(a.nxg - 2) || (unsigned)iy > (unsigned)(a.nyg - 2) ||
+                 (NDIM == 3 && (unsigned)iz > (unsigned)(a.nzg - 2)))) {
+        record_guard(a.cnt, ix, iy, iz, 1);
+        ok = false;
+    }
+    const size_t row = (size_t)a.nxg, plane = (size_t)a.nxg * a.nyg;
+    // 2D: no branch around the loads, so that both members' are in flight at
+    // once (46.9 -> 41.5 ms for 2e6 particles); a member without a push stands
+    // for cell 0, whose sums nobody reads.  3D, where a quarter of the members
+    // of a late chunk have none and a group's fourth lane has no sector: skipped
+    // (24.8 against 26.6 ms for 1e6 particles).
+    const uint32_t none = NDIM == 2 ? 0u : 0xffffffffu;
+    const uint32_t mine = ok ? (uint32_t)ix + (uint32_t)a.nxg * ((uint32_t)iy +
+                                                                  (uint32_t)a.nyg * (uint32_t)iz)
+                             : none;
+    const float *rec1 = a.rec1 + 8 * sub, *rec2 = a.rec2 + 8 * sub;
+    __syncwarp();   // the group has read its last sums
+#pragma unroll
+    for (int m = 0; m < G; ++m) {
+        const uint32_t base = __shfl_sync(0xffffffffu, mine, m, G);
+        const float fx = __shfl_sync(0xffffffffu, q.fx, m, G);
+        const float fy = __shfl_sync(0xffffffffu, q.fy, m, G);
+        const float fz = (NDIM == 3) ? __shfl_sync(0xffffffffu, q.fz, m, G) : 0.0f;
+        const float tm = a.time_interp ? __shfl_sync(0xffffffffu, rt, m, G) : 0.0f;
+        if (NDIM == 3 && (base == none || sub >= kSectors)) continue;
+        float s[8];
+#pragma unroll
+        for (int e = 0; e < 8; ++e) s[e] = 0.0f;
+        const float *r1 = rec1 + (size_t)R * base;
+        const float *r2 = rec2 + (size_t)R * base;
+#pragma unroll
+        for (int c = 0; c < kCorners; ++c) {
+            float wc = ((c & 1) ? fx : 1.0f - fx) * ((c & 2) ? fy : 1.0f - fy);
+            if (NDIM == 3) wc *= ((c & 4) ? fz : 1.0f - fz);
+            const size_t off = R * ((c & 1) + ((c & 2) ? row : 0) + ((c & 4) ? plane : 0));
+            float w1 = wc;
+            if (a.time_interp) w1 = wc * (1.0f - tm);
+            float g[8];
+            ld8(r1 + off, g);
+#pragma unroll
+            for (int e = 0; e < 8; ++e) s[e] = fmaf(g[e], w1, s[e]);
+            if (a.time_interp) {
+                const float w2 = wc * tm;
+                ld8(r2 + off, g);
+#pragma unroll
+                for (int e = 0; e < 8; ++e) s[e] = fmaf(g[e], w2, s[e]);
+            }
+        }
+        const int who = lane - sub + m;
+        float *to = buf + kGatherPlane * sub + 4 * ((who + sub) & 31);
+        *reinterpret_cast<float4 *>(to) = make_float4(s[0], s[1], s[2], s[3]);
+        if (NDIM == 3 && sub == 2)
+            buf[5 * kGatherPlane + who] = s[4];
+        else
+            *reinterpret_cast<float4 *>(to + kGatherPlane * kSectors) =
+                make_float4(s[4], s[5], s[6], s[7]);
+    }
+    __syncwarp();
+#pragma unroll
+    for (int v4 = 0; v4 < (NV + 3) / 4; ++v4) {
+        const int j = v4 >> 1, at = j + kSectors * (v4 & 1);
+        if (NDIM == 3 && v4 == 5) {
+            f[4 * v4] = buf[5 * kGatherPlane + lane];
+            continue;
+        }
+        const float4 g =
+            *reinterpret_cast<const float4 *>(buf + kGatherPlane * at + 4 * ((lane + j) & 31));
+        f[4 * v4] = g.x;
+        if (4 * v4 + 1 < NV) f[4 * v4 + 1] = g.y;
+        if (4 * v4 + 2 < NV) f[4 * v4 + 2] = g.z;
+        if (4 * v4 + 3 < NV) f[4 * v4 + 3] = g.w;
+    }
+    return ok;
 }
 
 // Gathers from the packed records in global memory; every position is
@@ -294,14 +398,11 @@ __device__ __forceinline__ bool in_acc_region(const MixedConsts &k, const Pos &q
 // kpara0 kperp_kpara |B|^((gamma-2)/3) (p/p0)^((5-gamma)/3) mu^2, with the
 // gradient terms T_i = kperp dkperp_i, A_i = kpara dkpara_i - kperp dkperp_i
 // in place of kperp dk_i and kpp dk_i.
-template <int NDIM, bool NLGC, class G>
-__device__ __forceinline__ bool push(const MixedRunArgs &a, const MixedConsts &k, const G &g,
-                                     const Pos &q, float p, float mu, float rt, bool fixed,
-                                     float &dt, uint32_t ctr, uint32_t ti, uint32_t ts, float &dX,
-                                     float &dY, float &dZ, float &dp) {
-    constexpr int NV = (NDIM == 2) ? 15 : 21;
-    float f[NV];
-    if (!g.template interp<NDIM, NV>(a, q, rt, f)) return false;
+template <int NDIM, bool NLGC>
+__device__ __forceinline__ void push_with(const MixedRunArgs &a, const MixedConsts &k,
+                                          const float *f, float p, float mu, bool fixed,
+                                          float &dt, uint32_t ctr, uint32_t ti, uint32_t ts,
+                                          float &dX, float &dY, float &dZ, float &dp) {
     // slots: 2D vx vy bx by bz dvx/dx dvy/dy dbx/dx dbx/dy dby/dx dby/dy dbz/dx dbz/dy db/dx db/dy
     //        3D vx vy vz bx by bz dvx/dx dvy/dy dvz/dz dbi/dj (9) db/dx db/dy db/dz
     constexpr int OB = (NDIM == 2) ? 2 : 3;
@@ -424,19 +525,32 @@ __device__ __forceinline__ bool push(const MixedRunArgs &a, const MixedConsts &k
         const float sq = skperp * ibxyn * sdt;
         dX = fmaf(dx_dt, dt, bxn * sp1 - bxn * bzn * sq * r[1] - byn * sq * r[2]) * k.idx;
         dY = fmaf(dy_dt, dt, byn * sp1 - byn * bzn * sq * r[1] + bxn * sq * r[2]) * k.idy;
-        dZ = fmaf(dz_dt, dt, bzn * sp1 + bxyn * skperp * r[1] * sdt) * k.idz;
+        dZ = fmaf(dz_dt, dt, fmaf(bzn, sp1, bxyn * skperp * r[1] * sdt)) * k.idz;
     }
     dp = dp_dt * dt;
+}
+
+template <int NDIM, bool NLGC, class G>
+__device__ __forceinline__ bool push(const MixedRunArgs &a, const MixedConsts &k, const G &g,
+                                     const Pos &q, float p, float mu, float rt, bool fixed,
+                                     float &dt, uint32_t ctr, uint32_t ti, uint32_t ts, float &dX,
+                                     float &dY, float &dZ, float &dp) {
+    constexpr int NV = (NDIM == 2) ? 15 : 21;
+    float f[NV];
+    if (!g.template interp<NDIM, NV>(a, q, rt, f)) return false;
+    push_with<NDIM, NLGC>(a, k, f, p, mu, fixed, dt, ctr, ti, ts, dX, dY, dZ, dp);
     return true;
 }
 
 // Resident 128-thread blocks per SM the register allocation targets (2D: 6
-// blocks = 80 registers, 3D: 5 blocks = 96 registers, measured best on GB300).
+// blocks = 80 registers, 3D: 4 blocks = 128 registers, measured best on GB300:
+// 2D, 5 to 7 blocks 41.9, 41.5, 44.2 ms for 2e6 particles; 3D, 3 to 6 blocks
+// 25.0, 24.8, 26.6, 28.6 ms for 1e6).
 #ifndef GPAT_MIXED_MINB_2D
 #define GPAT_MIXED_MINB_2D 6
 #endif
 #ifndef GPAT_MIXED_MINB_3D
-#define GPAT_MIXED_MINB_3D 5
+#define GPAT_MIXED_MINB_3D 4
 #endif
 
 // One particle's interval (or chunk of it): particle_mover_one_cycle's body
@@ -603,6 +717,189 @@ __device__ __forceinline__ uint32_t move_particle(const MixedRunArgs &a, const M
         P.nsteps_tracked[i] = 1;
         P.rng_ctr[i] = ctr;
     }
+    return pushes;
+}
+
+// (nsp + 1) % interval; a count inside the interval needs no division.
+__device__ __forceinline__ int next_nsp(int nsp, int interval) {
+    const int n = nsp + 1;
+    if ((unsigned)n < (unsigned)interval) return n;
+    return n == interval ? 0 : n % interval;
+}
+
+// move_particle with the gathers of a whole warp (interp_group): the loop turns
+// once per push of the warp, ordinary and landing pushes through the same
+// code, until no lane's particle has one left before its pause or the end of
+// the interval.  All lanes call; valid: the lane has a particle.
+template <int NDIM, bool NLGC>
+__device__ __forceinline__ uint32_t move_warp(const MixedRunArgs &a, const MixedConsts &k,
+                                              const DevParticles &P, int64_t i, bool valid,
+                                              bool &active, uint32_t limit, float *buf) {
+    constexpr int NV = (NDIM == 2) ? 15 : 21;
+    uint32_t pushes = 0;
+    active = false;
+    double x_in = 0.0, y_in = 0.0, z_in = 0.0, p_in = 0.0, t_in = 0.0;
+    const double *wp = P.weight + i;
+    Pos q = {0, 0, 0, 0.0f, 0.0f, 0.0f};
+    float p_f0 = 0.0f, tau_f0 = 0.0f, dt = 0.0f, mu = 0.0f;
+    double target_d = 0.0;
+    float target = 0.0f;                   // (float)target_d
+    int flag = 0, nsp = 0;
+    uint32_t ctr = 0, ti = 0, ts = 0;
+    if (valid) {
+        x_in = P.x[i]; y_in = P.y[i]; z_in = P.z[i];
+        p_in = P.p[i]; t_in = P.t[i];
+        cell_of(x_in, a.xmin, a.dx, q.cx, q.fx);
+        cell_of(y_in, a.ymin, a.dy, q.cy, q.fy);
+        if (NDIM == 3) cell_of(z_in, a.zmin, a.dz, q.cz, q.fz);
+        p_f0 = (float)p_in;
+        const double tau_in = t_in - a.t0;
+        tau_f0 = (float)tau_in;
+        dt = (float)P.dt[i];
+        flag = P.count_flag[i];
+        nsp = P.nsteps_pushed[i];
+        ctr = P.rng_ctr[i];
+        ti = (uint32_t)P.tag_injected[i];
+        ts = (uint32_t)P.tag_splitted[i];
+        if (NLGC) mu = (float)P.mu[i];
+        const double stepd = ceil(tau_in / a.dt_fine);
+        target_d = (stepd <= 0.0) ? a.dt_fine : stepd * a.dt_fine;
+        if (target_d > a.dtf) target_d = a.dtf;
+    }
+    const Pos q_in = q;
+    float z2 = 0.0f;                       // 2D out-of-plane drift, physical units
+    float p = p_f0, pc = 0.0f;
+    float tau = tau_f0, tc = 0.0f;
+    float landed_at = -1.0f;               // landed on the target, written as t0 + target_d
+    double landed_d = 0.0;
+    float uX = 0.0f, uY = 0.0f, uZ = 0.0f, uP = 0.0f;
+    if (valid) {
+        if (p < 0.0f && flag == 1) {
+            flag = 0;
+            atomic_add_fixed(&a.cnt->negp_hi, &a.cnt->negp_lo, *wp);
+        } else {
+            boundary<NDIM>(a, k, q, true, flag, wp);
+        }
+    }
+    // alive: in the box, with fine-step targets left in the interval
+    bool alive = valid && flag == 1 && target_d < a.limit;
+    target = (float)target_d;
+    bool paused = false;
+    float dtr = 0.0f;
+    for (;;) {
+        bool want = false, fixed = false;
+        while (alive && flag == 1) {
+            if (tau - tc < target) {
+                negp_or_boundary<NDIM>(a, k, q, p - pc, flag, wp);
+                if (flag != 1) break;
+                if (limit != 0 && pushes >= limit) {
+                    paused = true;   // between pushes: the next launch resumes from t
+                    alive = false;
+                    break;
+                }
+                if (pushes >= a.max_pushes) { set_status(a.cnt, kStatusStepLimit); alive = false; break; }
+                want = true;
+                break;
+            }
+            if (tau - tc > target) {
+                // Undo the overshooting push, redo it with dt = target - t.
+                advance(q.cx, q.fx, -uX);
+                advance(q.cy, q.fy, -uY);
+                // push_particle_2d's deltaz is local to it: the undo keeps the
+                // out-of-plane drift of the overshooting push.
+                if (NDIM == 3) advance(q.cz, q.fz, -uZ);
+                kadd(p, pc, -uP);
+                kadd(tau, tc, -dt);
+                dtr = target - (tau - tc);
+                if (dtr > 0.0f) {
+                    nsp = nsp - 1;
+                    want = true;
+                    fixed = true;
+                    break;
+                }
+                negp_or_boundary<NDIM>(a, k, q, p - pc, flag, wp);
+            } else if (tau - tc == target) {
+                landed_at = 1.0f;      // reached the target without overshoot
+                landed_d = target_d;
+            }
+            target_d = target_d + a.dt_fine;
+            target = (float)target_d;
+            alive = target_d < a.limit;
+        }
+        if (!__any_sync(0xffffffffu, want)) break;
+        float f[NV];
+        const bool ok = interp_group<NDIM, NV>(a, q, tau * k.inv_dtf, want, buf, f);
+        if (!want) continue;
+        if (!ok) {
+            flag = 0;
+            alive = false;
+            continue;
+        }
+        const float pe = p - pc;
+        float dp;
+        auto push_on = [&](const bool fix) {
+            float step = fix ? dtr : dt;
+            push_with<NDIM, NLGC>(a, k, f, pe, mu, fix, step, ctr, ti, ts, uX, uY, uZ, dp);
+            ++ctr;
+            ++pushes;
+            advance(q.cx, q.fx, uX);
+            advance(q.cy, q.fy, uY);
+            if (NDIM == 3) advance(q.cz, q.fz, uZ); else z2 += uZ;
+            if (!fix) {
+                dt = step;
+                kadd(tau, tc, dt);
+            }
+            if (a.acc_region_flag == 1 && !in_acc_region<NDIM>(k, q)) dp = 0.0f;
+            if (pe + dp < k.pfloor) { dp = k.pfloor - pe; p = k.pfloor; pc = 0.0f; }
+            else kadd(p, pc, dp);
+            uP = dp;
+            nsp = next_nsp(nsp, a.nsteps_interval);
+            if (fix) {
+                tau = target; tc = 0.0f;
+                landed_at = 1.0f;
+                landed_d = target_d;
+                negp_or_boundary<NDIM>(a, k, q, p - pc, flag, wp);
+                target_d = target_d + a.dt_fine;
+                target = (float)target_d;
+                alive = target_d < a.limit;
+            } else {
+                landed_at = -1.0f;
+                if (!(fabsf(tau) < 1e30f) || !(fabsf(p) < 1e30f) || !(q.fx <= 1.0f) ||
+                    !(q.fy <= 1.0f) || !(q.fz <= 1.0f)) {
+                    set_status(a.cnt, kStatusNonFinite);
+                    flag = 0;
+                    alive = false;
+                }
+            }
+        };
+        // 3D: one copy of the code, which fills the instruction cache; 2D: one
+        // for each kind of push
+        if (NDIM == 3) push_on(fixed);
+        else if (fixed) push_on(true);
+        else push_on(false);
+    }
+    if (!valid) return 0;
+    if (flag == 1 && !paused) boundary<NDIM>(a, k, q, false, flag, wp);
+    active = paused;
+    // Write back input + change, computed in FP64.
+    const double dcx = (double)(q.cx - q_in.cx) + ((double)q.fx - (double)q_in.fx);
+    const double dcy = (double)(q.cy - q_in.cy) + ((double)q.fy - (double)q_in.fy);
+    P.x[i] = x_in + dcx * a.dx;
+    P.y[i] = y_in + dcy * a.dy;
+    if (NDIM == 3) {
+        const double dcz = (double)(q.cz - q_in.cz) + ((double)q.fz - (double)q_in.fz);
+        P.z[i] = z_in + dcz * a.dz;
+    } else if (z2 != 0.0f) {
+        P.z[i] = z_in + (double)z2;
+    }
+    P.p[i] = p_in + (((double)p - (double)pc) - (double)p_f0);
+    P.t[i] = landed_at >= 0.0f ? a.t0 + landed_d
+                               : t_in + (((double)tau - (double)tc) - (double)tau_f0);
+    P.dt[i] = (double)dt;
+    P.count_flag[i] = (int8_t)flag;
+    P.nsteps_pushed[i] = nsp;
+    P.nsteps_tracked[i] = 1;
+    P.rng_ctr[i] = ctr;
     return pushes;
 }
 

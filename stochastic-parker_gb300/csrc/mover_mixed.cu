@@ -59,14 +59,12 @@ template <int NDIM, bool NLGC>
 __global__ void __launch_bounds__(128, NDIM == 2 ? GPAT_MIXED_MINB_2D : GPAT_MIXED_MINB_3D)
     mover_mixed_kernel(const MixedRunArgs a, const MixedConsts k, const DevParticles P,
                        const int64_t n) {
+    __shared__ __align__(16) float gather[4][kGatherBuf<NDIM>];
     const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    bool active = false, exited = false;
-    uint32_t pushes = 0;
-    if (i < n) {
-        pushes = move_particle<NDIM, NLGC>(a, k, P, i, active, GlobalGather{}, a.chunk_pushes,
-                                           exited);
-        if (a.pause) a.pause[i] = active ? 1 : 0;
-    }
+    bool active = false;
+    const uint32_t pushes = move_warp<NDIM, NLGC>(a, k, P, i, i < n, active, a.chunk_pushes,
+                                                  gather[threadIdx.x >> 5]);
+    if (i < n && a.pause) a.pause[i] = active ? 1 : 0;
     add_warp_counters(a.cnt, pushes, active, nullptr);
 }
 
@@ -84,14 +82,12 @@ __global__ void __launch_bounds__(128, NDIM == 2 ? GPAT_MIXED_MINB_2D : GPAT_MIX
     mma_mlp::SmemInf &S = *reinterpret_cast<mma_mlp::SmemInf *>(smem_raw);
     mma_mlp::load_smem(L.w16, S, false);
     __syncthreads();
+    __shared__ __align__(16) float gather[4][kGatherBuf<NDIM>];
     const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    bool active = false, exited = false;
-    uint32_t pushes = 0;
-    if (i < n) {
-        pushes = move_particle<NDIM, NLGC>(a, k, P, i, active, GlobalGather{}, a.chunk_pushes,
-                                           exited);
-        if (a.pause) a.pause[i] = active ? 1 : 0;
-    }
+    bool active = false;
+    const uint32_t pushes = move_warp<NDIM, NLGC>(a, k, P, i, i < n, active, a.chunk_pushes,
+                                                  gather[threadIdx.x >> 5]);
+    if (i < n && a.pause) a.pause[i] = active ? 1 : 0;
     add_warp_counters(a.cnt, pushes, active, nullptr);
     const bool fin = i < n && !active && P.count_flag[i] == 1;
     if (!__any_sync(0xffffffffu, fin)) return;
@@ -129,6 +125,7 @@ __global__ void __launch_bounds__(128, MINB)
                              const unsigned long long *run_n, unsigned long long *tile_counter,
                              const int grab, unsigned long long *nactive_total) {
     __shared__ long long s_tile;
+    __shared__ __align__(16) float gather[4][kGatherBuf<NDIM>];
     const long long total = tile_prefix[nruns];
     for (;;) {
         __syncthreads();
@@ -146,11 +143,10 @@ __global__ void __launch_bounds__(128, MINB)
             }
             const BatchRun &d = c_batch_runs[lo];
             const int64_t i = (t - tile_prefix[lo]) * 128 + threadIdx.x;
-            bool active = false, exited = false;
-            uint32_t pushes = 0;
-            if (i < (int64_t)run_n[lo])
-                pushes = move_particle<NDIM, NLGC>(d.a, d.k, d.P[parity], i, active, GlobalGather{},
-                                                  d.a.chunk_pushes, exited);
+            bool active = false;
+            const uint32_t pushes =
+                move_warp<NDIM, NLGC>(d.a, d.k, d.P[parity], i, i < (int64_t)run_n[lo], active,
+                                      d.a.chunk_pushes, gather[threadIdx.x >> 5]);
             add_warp_counters(d.a.cnt, pushes, active, nactive_total);
         }
     }
