@@ -69,6 +69,9 @@ struct gpat_handle {
     // and the bins of that binning
     uint8_t *pause = nullptr;
     int64_t pause_cap = 0;
+    // distributions: bins, then weights and counts on their way to the host
+    unsigned long long *bins_ws = nullptr;
+    size_t bins_ws_bytes = 0;
     // FP64 mover: the order its lanes take the particles in
     uint32_t *work = nullptr;
     int64_t work_cap = 0;
@@ -760,6 +763,7 @@ int gpat_destroy(gpat_handle_t *h) {
     if (h->tile_dev) cudaFree(h->tile_dev);
     if (h->pause) cudaFree(h->pause);
     if (h->work) cudaFree(h->work);
+    if (h->bins_ws) cudaFree(h->bins_ws);
     if (h->learn_dev) cudaFree(h->learn_dev);
     if (h->fresh_dev) cudaFree(h->fresh_dev);
     if (h->tile_ovf) cudaFree(h->tile_ovf);
@@ -1721,6 +1725,58 @@ int gpat_local_distribution_dims(gpat_handle_t *h, const gpat_local_dist_t *spec
     return GPAT_OK;
 }
 
+extern "C++" {
+// Runs a binning (wide: launch_local_dist's words, otherwise zeroed (count, whi,
+// wlo) triples) into a device buffer, turns it into weights and counts there,
+// kBinsOut at a time, and copies those to f and c (either may be NULL).  The
+// handle keeps a buffer of up to kBinsKept bytes.
+template <class Launch>
+static int run_bins(gpat_handle_t *h, size_t nbins, bool wide, Launch launch, double *f,
+                    uint64_t *c) {
+    if (nbins > ((size_t)1 << 31)) return fail(h, GPAT_ERR_ARG, "distribution too large");
+    CK(cudaSetDevice(h->device));
+    constexpr size_t kBinsKept = (size_t)64 << 20, kBinsOut = (size_t)1 << 22;
+    const size_t words = wide ? local_dist_words(nbins) : 3 * nbins;
+    const size_t per = words / std::max<size_t>(nbins, 1), part = std::min(nbins, kBinsOut);
+    const size_t bytes = sizeof(unsigned long long) * (words + 2 * part);
+    unsigned long long *bins = h->bins_ws;
+    const bool own = bytes <= kBinsKept;
+    if (!own || bytes > h->bins_ws_bytes) {
+        if (own && h->bins_ws) {
+            CK(cudaFree(h->bins_ws));
+            h->bins_ws = nullptr;
+            h->bins_ws_bytes = 0;
+        }
+        if (cudaMalloc((void **)&bins, bytes) != cudaSuccess) {
+            cudaGetLastError();
+            return fail(h, GPAT_ERR_OOM, "distribution does not fit in device memory");
+        }
+        if (own) {
+            h->bins_ws = bins;
+            h->bins_ws_bytes = bytes;
+        }
+    }
+    double *df = reinterpret_cast<double *>(bins + words);
+    unsigned long long *dc = bins + words + part;
+    cudaError_t e = cudaSuccess;
+    if (!wide) e = cudaMemsetAsync(bins, 0, sizeof(unsigned long long) * words, h->stream);
+    if (e == cudaSuccess) e = launch(bins);
+    for (size_t b = 0; b < nbins && e == cudaSuccess; b += kBinsOut) {
+        const size_t m = std::min(kBinsOut, nbins - b);
+        e = launch_bins_out(bins + per * b, m, (int)per, df, dc, h->stream);
+        if (e == cudaSuccess && f)
+            e = cudaMemcpyAsync(f + b, df, sizeof(double) * m, cudaMemcpyDeviceToHost, h->stream);
+        if (e == cudaSuccess && c)
+            e = cudaMemcpyAsync(c + b, dc, sizeof(uint64_t) * m, cudaMemcpyDeviceToHost, h->stream);
+    }
+    const cudaError_t es = cudaStreamSynchronize(h->stream);
+    if (!own) cudaFree(bins);
+    if (e == cudaSuccess) e = es;
+    if (e != cudaSuccess) return fail(h, GPAT_ERR_CUDA, cudaGetErrorString(e));
+    return GPAT_OK;
+}
+}  // extern "C++"
+
 int gpat_calc_local_distribution(gpat_handle_t *h, const gpat_local_dist_t *spec, double *flocal,
                                  uint64_t *counts) {
     if (!h) return GPAT_ERR_ARG;
@@ -1729,27 +1785,9 @@ int gpat_calc_local_distribution(gpat_handle_t *h, const gpat_local_dist_t *spec
     if (rc) return rc;
     const size_t nbins = (size_t)a.nmu * a.npb * a.nrx * a.nry * a.nrz;
     if (nbins > ((size_t)1 << 31)) return fail(h, GPAT_ERR_ARG, "local distribution too large");
-    CK(cudaSetDevice(h->device));
-    unsigned long long *bins = nullptr;
-    std::vector<unsigned long long> b;
-    try {
-        b.resize(3 * nbins);
-    } catch (const std::bad_alloc &) {
-        return fail(h, GPAT_ERR_OOM, "local distribution does not fit in host memory");
-    }
-    CK(cudaMallocAsync((void **)&bins, sizeof(unsigned long long) * 3 * nbins, h->stream));
-    cudaError_t e = launch_local_dist(h->P[h->cur], h->n, a, bins, nbins, h->stream);
-    if (e == cudaSuccess)
-        e = cudaMemcpyAsync(b.data(), bins, sizeof(unsigned long long) * b.size(),
-                            cudaMemcpyDeviceToHost, h->stream);
-    cudaFreeAsync(bins, h->stream);
-    if (e == cudaSuccess) e = cudaStreamSynchronize(h->stream);
-    if (e != cudaSuccess) return fail(h, GPAT_ERR_CUDA, cudaGetErrorString(e));
-    for (size_t i = 0; i < nbins; ++i) {
-        if (counts) counts[i] = b[3 * i];
-        if (flocal) flocal[i] = fixed_to_double(b[3 * i + 1], b[3 * i + 2]);
-    }
-    return GPAT_OK;
+    return run_bins(h, nbins, true, [&](unsigned long long *bins) {
+        return launch_local_dist(h->P[h->cur], h->n, a, bins, nbins, h->stream);
+    }, flocal, counts);
 }
 
 int gpat_calc_escaped_distributions(gpat_handle_t *h, double *fescaped, uint64_t *counts) {
@@ -1770,36 +1808,6 @@ int gpat_calc_escaped_distributions(gpat_handle_t *h, double *fescaped, uint64_t
     return GPAT_OK;
 }
 
-extern "C++" {
-// Runs a (count, whi, wlo) binning into a temporary device buffer and
-// unpacks it into counts / weights (either may be NULL).
-template <class Launch>
-static int run_bins(gpat_handle_t *h, size_t nbins, Launch launch, double *f, uint64_t *c) {
-    if (nbins > ((size_t)1 << 31)) return fail(h, GPAT_ERR_ARG, "distribution too large");
-    CK(cudaSetDevice(h->device));
-    unsigned long long *bins = nullptr;
-    std::vector<unsigned long long> b;
-    try {
-        b.resize(3 * nbins);
-    } catch (const std::bad_alloc &) {
-        return fail(h, GPAT_ERR_OOM, "distribution does not fit in host memory");
-    }
-    CK(cudaMallocAsync((void **)&bins, sizeof(unsigned long long) * 3 * nbins, h->stream));
-    cudaError_t e = cudaMemsetAsync(bins, 0, sizeof(unsigned long long) * 3 * nbins, h->stream);
-    if (e == cudaSuccess) e = launch(bins);
-    if (e == cudaSuccess)
-        e = cudaMemcpyAsync(b.data(), bins, sizeof(unsigned long long) * b.size(),
-                            cudaMemcpyDeviceToHost, h->stream);
-    cudaFreeAsync(bins, h->stream);
-    if (e == cudaSuccess) e = cudaStreamSynchronize(h->stream);
-    if (e != cudaSuccess) return fail(h, GPAT_ERR_CUDA, cudaGetErrorString(e));
-    for (size_t i = 0; i < nbins; ++i) {
-        if (c) c[i] = b[3 * i];
-        if (f) f[i] = fixed_to_double(b[3 * i + 1], b[3 * i + 2]);
-    }
-    return GPAT_OK;
-}
-
 static MuDistArgs mu_args(const gpat_handle_t *h, int nmu, int by_face) {
     MuDistArgs a;
     a.pmin = h->prm.pmin;
@@ -1812,7 +1820,6 @@ static MuDistArgs mu_args(const gpat_handle_t *h, int nmu, int by_face) {
     a.by_face = by_face;
     return a;
 }
-}  // extern "C++"
 
 int gpat_calc_particle_distributions_mu(gpat_handle_t *h, int32_t nmu, double *fglobal,
                                         uint64_t *counts) {
@@ -1820,7 +1827,7 @@ int gpat_calc_particle_distributions_mu(gpat_handle_t *h, int32_t nmu, double *f
     if (nmu < 1) return fail(h, GPAT_ERR_ARG, "nmu must be >= 1");
     const MuDistArgs a = mu_args(h, nmu, 0);
     const size_t nbins = (size_t)nmu * (size_t)a.npp;
-    return run_bins(h, nbins, [&](unsigned long long *bins) {
+    return run_bins(h, nbins, false, [&](unsigned long long *bins) {
         return launch_mu_dist(h->P[h->cur], h->n, a, bins, nbins, h->stream);
     }, fglobal, counts);
 }
@@ -1831,7 +1838,7 @@ int gpat_calc_escaped_distributions_mu(gpat_handle_t *h, int32_t nmu, double *fe
     if (nmu < 1) return fail(h, GPAT_ERR_ARG, "nmu must be >= 1");
     const MuDistArgs a = mu_args(h, nmu, 1);
     const size_t nbins = (size_t)nmu * (size_t)a.npp * 2 * (size_t)h->prm.ndim;
-    return run_bins(h, nbins, [&](unsigned long long *bins) {
+    return run_bins(h, nbins, false, [&](unsigned long long *bins) {
         return launch_mu_dist(h->E, h->ne, a, bins, nbins, h->stream);
     }, fescaped, counts);
 }
@@ -1851,7 +1858,7 @@ int gpat_calc_local_escaped_distribution(gpat_handle_t *h, const gpat_local_dist
     uint64_t *c[3] = {cx, cy, cz};
     for (int face = 0; face < 3; ++face) {
         if (!sizes[face] || (!f[face] && !c[face])) continue;
-        rc = run_bins(h, sizes[face], [&](unsigned long long *bins) {
+        rc = run_bins(h, sizes[face], false, [&](unsigned long long *bins) {
             unsigned long long *b[3] = {nullptr, nullptr, nullptr};
             b[face] = bins;
             return launch_local_escaped(h->E, h->ne, a, b[0], b[1], b[2], h->stream);

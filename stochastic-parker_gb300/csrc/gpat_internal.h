@@ -395,15 +395,22 @@ struct LocalDistArgs {
     int ndim, spherical, nonuniform, rx, ry, rz, nxg, nyg, nzg;
     const double *xpos, *ypos, *zpos;
 };
-// bins: (count, whi, wlo) per flocal element, zeroed here.
+// bins: local_dist_words(nbins) words, zeroed here; launch_bins_out (wide) reads
+// them.
+size_t local_dist_words(size_t nbins);
 cudaError_t launch_local_dist(const DevParticles &P, int64_t n, const LocalDistArgs &a,
                               unsigned long long *bins, size_t nbins, cudaStream_t s);
+// Bins as doubles (weights) and counts.  words per bin: 3, (count, whi, wlo), or
+// launch_local_dist's local_dist_words(1).
+cudaError_t launch_bins_out(const unsigned long long *bins, size_t nbins, int words, double *f,
+                            unsigned long long *c, cudaStream_t s);
 // Local escaped distributions into the per-face (count, whi, wlo) arrays
 // fx, fy, fz (zeroed by the caller; nullptr skips a face).
 cudaError_t launch_local_escaped(const DevParticles &P, int64_t n, const LocalDistArgs &a,
                                  unsigned long long *fx, unsigned long long *fy,
                                  unsigned long long *fz, cudaStream_t s);
-// Global (or, with by_face, escaped) distribution with pitch-angle bins.
+// Global (or, with by_face, escaped) distribution with pitch-angle bins (nmu 0:
+// one bin for every pitch angle in [-1, 1]).
 struct MuDistArgs {
     double pmin, pmax, pmin_log, dp_log, dmu;
     int npp, nmu, by_face;

@@ -1,8 +1,10 @@
 // Particle-set kernels around the mover: injection, stable removal
 // (remove_particles), splitting (split_particle), the global f(p) histogram
 // (calc_particle_distributions) and the quick_check reductions.
+#include <algorithm>
 #include <cfloat>
 
+#include "bins_common.cuh"
 #include "cell_index.cuh"
 #include "device_common.cuh"
 #include "grid_common.cuh"
@@ -546,82 +548,135 @@ __global__ void __launch_bounds__(kScanThreads) tile_scatter_kernel(
 }
 
 // ---------------------------------------------------------------------------
-// Global f(p) histogram: block-private shared bins (count, weight hi, lo),
-// warp-aggregated by bin with __match_any_sync, exact 128-bit weights.
+// Global f(p), without or with pitch-angle bins (calc_particle_distributions
+// :738-780, calc_escaped_distributions :949-957): fglobal(nmu, npp) or, with
+// by_face, fescaped(nmu, npp, |count_flag|); the particle's own weight.  p ==
+// pmax and mu == 1 index past the last bin in the reference and are dropped.
 // ---------------------------------------------------------------------------
-__global__ void __launch_bounds__(256) histogram_kernel(const DevParticles P, int64_t n, int npp,
-                                                        double pmin, double pmax, double pmin_log,
-                                                        double dp_log, unsigned long long *bins) {
-    extern __shared__ unsigned long long sh[];  // 3 * npp
-    for (int b = threadIdx.x; b < 3 * npp; b += blockDim.x) sh[b] = 0ull;
+struct MuBins {
+    MuDistArgs a;
+    LogBins lp;
+    EvenBins mu;
+};
+
+__device__ __forceinline__ int64_t mu_bin(const DevParticles &P, int64_t i, const MuBins &g) {
+    const MuDistArgs &a = g.a;
+    const double p = P.p[i], mu = P.mu[i];
+    if (!less(a.pmin, p) || less(a.pmax, p) || !within_one(mu)) return -1;
+    const int ip = log_bin(p, g.lp) + 1;
+    const int imu = a.nmu == 0 ? 1 : even_bin(mu, g.mu) + 1;
+    const int nmu = a.nmu == 0 ? 1 : a.nmu;
+    if (ip < 1 || ip > a.npp || imu < 1 || imu > nmu) return -1;
+    int64_t face = 0;
+    if (a.by_face) {
+        const int flag = P.count_flag[i];
+        if (flag >= 0 || flag < -6) return -1;
+        face = -flag - 1;
+    }
+    return (int64_t)(imu - 1) + (int64_t)nmu * ((int64_t)(ip - 1) + (int64_t)a.npp * face);
+}
+
+// Block-private bins in shared memory, a count and the limbs of the weights
+// each, added to the global (count, weight hi, lo) triples at the end and
+// before a word could overflow.  HBM streaming, 24 B per particle; with FP64
+// logarithms, 64-bit bins and a merge of equal bins in the warp it took 384 us
+// for 4e6 particles (npp 128) and 485 us with 8 pitch-angle bins.
+constexpr int kBinWords = 1 + kLimbs;
+
+__global__ void __launch_bounds__(256) bins_shared_kernel(const DevParticles P, int64_t n,
+                                                          const MuBins g, int nbins,
+                                                          unsigned long long *bins) {
+    extern __shared__ unsigned int words[];   // kBinWords * nbins
+    for (int b = threadIdx.x; b < kBinWords * nbins; b += blockDim.x) words[b] = 0u;
     __syncthreads();
     const int64_t stride = (int64_t)gridDim.x * blockDim.x;
-    const int64_t start = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     const int64_t iters = (n + stride - 1) / stride;
     for (int64_t it = 0; it < iters; ++it) {
-        const int64_t i = start + it * stride;
-        int bin = -1;
-        unsigned long long wh = 0, wl = 0;
+        const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x + it * stride;
         if (i < n) {
-            const double p = P.p[i], mu = P.mu[i];
-            if (p > pmin && p <= pmax && mu >= -1.0 && mu <= 1.0) {
-                const int ip = (int)floor((log10(p) - pmin_log) / dp_log);
-                if (ip >= 0 && ip < npp) {
-                    bin = ip;
-                    fixed_split(P.weight[i], wh, wl);
-                }
+            const int64_t b = mu_bin(P, i, g);
+            if (b >= 0) {
+                unsigned long long h, l;
+                fixed_parts(P.weight[i], h, l);
+                unsigned int *w = words + kBinWords * b;
+                atomicAdd(w, 1u);
+                limbs_add(w + 1, h, l);
             }
         }
-        const unsigned grp = __match_any_sync(0xffffffffu, bin);
-        const int leader = __ffs(grp) - 1;
-        unsigned long long sh_h = 0, sh_l = 0;
-        unsigned m = grp;
-        while (m) {
-            const int src = __ffs(m) - 1;
-            m &= m - 1;
-            const unsigned long long oh = __shfl_sync(grp, wh, src);
-            const unsigned long long ol = __shfl_sync(grp, wl, src);
-            add_u128(sh_h, sh_l, oh, ol);
+        if ((it & 255) == 255 || it == iters - 1) {   // at most 65536 weights a word
+            __syncthreads();
+            for (int b = threadIdx.x; b < nbins; b += blockDim.x) {
+                unsigned int *w = words + kBinWords * b;
+                if (w[0] == 0u) continue;
+                unsigned long long h, l;
+                limbs_sum(w + 1, h, l);
+                atomicAdd(&bins[3 * b], (unsigned long long)w[0]);
+                atomic_add_u128(&bins[3 * b + 1], &bins[3 * b + 2], h, l);
+                for (int k = 0; k < kBinWords; ++k) w[k] = 0u;
+            }
+            __syncthreads();
         }
-        if (bin >= 0 && (int)(threadIdx.x & 31) == leader) {
-            atomicAdd(&sh[3 * bin], (unsigned long long)__popc(grp));
-            atomic_add_u128(&sh[3 * bin + 1], &sh[3 * bin + 2], sh_h, sh_l);
-        }
-    }
-    __syncthreads();
-    for (int b = threadIdx.x; b < npp; b += blockDim.x) {
-        if (sh[3 * b]) atomicAdd(&bins[3 * b], sh[3 * b]);
-        atomic_add_u128(&bins[3 * b + 1], &bins[3 * b + 2], sh[3 * b + 1], sh[3 * b + 2]);
     }
 }
 
 // ---------------------------------------------------------------------------
 // quick_check: exact sums of weight and dt, min/max dt (positive doubles
-// order like their bit patterns).
+// order like their bit patterns).  HBM streaming, 16 B per particle; one set of
+// atomics per block and four blocks per SM, since all go to the same few
+// addresses (one set per warp of 2048 blocks took 100 us).
 // ---------------------------------------------------------------------------
 __global__ void __launch_bounds__(256) quick_check_kernel(const DevParticles P, int64_t n,
                                                           DevCounters *cnt) {
     unsigned long long wh = 0, wl = 0, th = 0, tl = 0;
     double mn = 1.0, mx = 0.0;
     const int64_t stride = (int64_t)gridDim.x * blockDim.x;
-    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += stride) {
-        unsigned long long h, l;
-        fixed_split(P.weight[i], h, l);
-        add_u128(wh, wl, h, l);
-        const double dt = P.dt[i];
-        fixed_split(dt, h, l);
-        add_u128(th, tl, h, l);
-        if (dt < mn) mn = dt;
-        if (dt > mx) mx = dt;
-    }
-    warp_sum_u128(wh, wl);
-    warp_sum_u128(th, tl);
+    for (int64_t i0 = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i0 < n; i0 += 4 * stride) {
+        double w[4], t[4];
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-        mn = fmin(mn, __shfl_xor_sync(0xffffffffu, mn, o));
-        mx = fmax(mx, __shfl_xor_sync(0xffffffffu, mx, o));
+        for (int k = 0; k < 4; ++k) {   // four loads of each in flight; past the end: nothing
+            const int64_t i = i0 + k * stride;
+            w[k] = i < n ? P.weight[i] : 0.0;
+            t[k] = i < n ? P.dt[i] : mn;
+        }
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+            unsigned long long h, l;
+            fixed_parts(w[k], h, l);
+            add_u128(wh, wl, h, l);
+            if (i0 + k * stride >= n) break;
+            fixed_parts(t[k], h, l);
+            add_u128(th, tl, h, l);
+            if (less(t[k], mn)) mn = t[k];
+            if (less(mx, t[k])) mx = t[k];
+        }
     }
-    if ((threadIdx.x & 31) == 0) {
+    __shared__ unsigned long long sums[8][4];
+    __shared__ double ends[8][2];
+    for (int level = 0; level < 2; ++level) {
+        warp_sum_u128(wh, wl);
+        warp_sum_u128(th, tl);
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) {
+            const double on = __shfl_xor_sync(0xffffffffu, mn, o);
+            const double ox = __shfl_xor_sync(0xffffffffu, mx, o);
+            if (less(on, mn)) mn = on;
+            if (less(mx, ox)) mx = ox;
+        }
+        if (level == 1) break;
+        const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+        if (lane == 0) {
+            sums[warp][0] = wh; sums[warp][1] = wl; sums[warp][2] = th; sums[warp][3] = tl;
+            ends[warp][0] = mn; ends[warp][1] = mx;
+        }
+        __syncthreads();
+        if (warp > 0) return;
+        const bool in = lane < 8;
+        wh = in ? sums[lane][0] : 0ull; wl = in ? sums[lane][1] : 0ull;
+        th = in ? sums[lane][2] : 0ull; tl = in ? sums[lane][3] : 0ull;
+        mn = in ? ends[lane][0] : 1.0;
+        mx = in ? ends[lane][1] : 0.0;
+    }
+    if (threadIdx.x == 0) {
         atomic_add_u128(&cnt->wsum_hi, &cnt->wsum_lo, wh, wl);
         atomic_add_u128(&cnt->dtsum_hi, &cnt->dtsum_lo, th, tl);
         if (mn >= 0.0)
@@ -1034,16 +1089,15 @@ cudaError_t launch_sync_tracked(const TrackArgs &trk, cudaStream_t s) {
 
 cudaError_t launch_histogram(const DevParticles &P, int64_t n, int npp, double pmin, double pmax,
                              unsigned long long *bins, cudaStream_t s) {
-    cudaError_t e = cudaMemsetAsync(bins, 0, sizeof(unsigned long long) * 3 * (size_t)npp, s);
-    if (e != cudaSuccess || n <= 0) return e;
-    const double pmin_log = log10(pmin), pmax_log = log10(pmax);
-    const double dp_log = (pmax_log - pmin_log) / npp;
-    int64_t blocks = (n + 255) / 256;
-    if (blocks > 4096) blocks = 4096;
-    const size_t shmem = sizeof(unsigned long long) * 3 * (size_t)npp;
-    histogram_kernel<<<(unsigned)blocks, 256, shmem, s>>>(P, n, npp, pmin, pmax, pmin_log, dp_log,
-                                                          bins);
-    return cudaGetLastError();
+    MuDistArgs a{};
+    a.pmin = pmin;
+    a.pmax = pmax;
+    a.pmin_log = log10(pmin);
+    a.dp_log = (log10(pmax) - a.pmin_log) / npp;
+    a.dmu = 1.0;
+    a.npp = npp;
+    a.nmu = 0;   // one bin for all pitch angles
+    return launch_mu_dist(P, n, a, bins, (size_t)npp, s);
 }
 
 // The bins of particle i for one local-distribution parameter set
@@ -1054,8 +1108,25 @@ struct LocalBin {
     double w;
 };
 
+// The parameter set with what the bins' cheaper forms need.
+struct LocalBins {
+    LocalDistArgs a;
+    LogBins lp;
+    EvenBins x, y, z, mu;
+};
+
+LocalBins make_local_bins(const LocalDistArgs &a) {
+    return LocalBins{a,
+                     make_log_bins(a.pmin_log, a.dp_log),
+                     make_even_bins(a.xmin, a.dxd),
+                     make_even_bins(a.ymin, a.dyd),
+                     make_even_bins(a.zmin, a.dzd),
+                     make_even_bins(-1.0, a.dmu)};
+}
+
 __device__ __forceinline__ LocalBin local_bin(const DevParticles &P, int64_t i,
-                                              const LocalDistArgs &a) {
+                                              const LocalBins &g) {
+    const LocalDistArgs &a = g.a;
     LocalBin b;
     const double p = P.p[i], mu = P.mu[i];
     int ix, iy, iz;
@@ -1068,13 +1139,13 @@ __device__ __forceinline__ LocalBin local_bin(const DevParticles &P, int64_t i,
         iz = (a.ndim == 3) ? (grid_count(a.zpos, a.nzg, P.z[i]) - 1) / a.rz + 1
                            : (int)floor((P.z[i] - a.zmin) / a.dzd) + 1;
     } else {
-        ix = (int)floor((P.x[i] - a.xmin) / a.dxd) + 1;
-        iy = (int)floor((P.y[i] - a.ymin) / a.dyd) + 1;
-        iz = (int)floor((P.z[i] - a.zmin) / a.dzd) + 1;
+        ix = even_bin(P.x[i], g.x) + 1;
+        iy = even_bin(P.y[i], g.y) + 1;
+        iz = even_bin(P.z[i], g.z) + 1;
     }
     b.ix = ix; b.iy = iy; b.iz = iz;
-    b.ip = (int)floor((log10(p) - a.pmin_log) / a.dp_log) + 1;
-    b.imu = (int)floor((mu + 1.0) / a.dmu) + 1;
+    b.ip = log_bin(p, g.lp) + 1;
+    b.imu = even_bin(mu, g.mu) + 1;
     double w = P.weight[i];
     if (a.spherical) {
         // F = f p^2 r^2 (sin theta from 2D on), diagnostics.f90:765-772
@@ -1091,14 +1162,20 @@ __device__ __forceinline__ void bin_add(unsigned long long *bins, size_t e, doub
     atomic_add_fixed(b + 1, b + 2, w);
 }
 
-// Local distributions (calc_particle_distributions, diagnostics.f90:782-878):
-// one (count, weight hi, lo) triple per flocal element.
+// Local distributions (calc_particle_distributions, diagnostics.f90:782-878).
+// WIDE: kWideWords 64-bit words per flocal element, a count and the weight's four
+// 32-bit limbs, each added without a returned value or a carry; otherwise the
+// (count, weight hi, lo) triple.
+constexpr int kWideWords = 5;
+
+template <bool WIDE>
 __global__ void __launch_bounds__(256) local_dist_kernel(const DevParticles P, int64_t n,
-                                                         const LocalDistArgs a,
+                                                         const LocalBins g,
                                                          unsigned long long *bins) {
+    const LocalDistArgs &a = g.a;
     const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
-    const LocalBin b = local_bin(P, i, a);
+    const LocalBin b = local_bin(P, i, g);
     if (b.ix < 1 || b.ix > a.nrx || b.iy < 1 || b.iy > a.nry || b.iz < 1 || b.iz > a.nrz) return;
     if (!(b.ip > 0 && b.ip < a.npb) || b.imu < 1 || b.imu > a.nmu) return;
     const size_t e = (size_t)(b.imu - 1) +
@@ -1106,7 +1183,41 @@ __global__ void __launch_bounds__(256) local_dist_kernel(const DevParticles P, i
                                       (size_t)a.npb * ((size_t)(b.ix - 1) +
                                                        (size_t)a.nrx * ((size_t)(b.iy - 1) +
                                                                         (size_t)a.nry * (b.iz - 1))));
-    bin_add(bins, e, b.w);
+    if (WIDE) {
+        unsigned long long h, l, *w = bins + kWideWords * e;
+        fixed_parts(b.w, h, l);
+        atomicAdd(w, 1ull);
+        if (l & 0xffffffffull) atomicAdd(w + 1, l & 0xffffffffull);
+        if (l >> 32) atomicAdd(w + 2, l >> 32);
+        if (h & 0xffffffffull) atomicAdd(w + 3, h & 0xffffffffull);
+        if (h >> 32) atomicAdd(w + 4, h >> 32);
+    } else {
+        bin_add(bins, e, b.w);
+    }
+}
+
+// Bins of WORDS words (kWideWords, or 3: the triples) -> weights as doubles
+// and counts.
+template <int WORDS>
+__global__ void __launch_bounds__(256) bins_out_kernel(const unsigned long long *bins,
+                                                       size_t nbins, double *f,
+                                                       unsigned long long *c) {
+    const size_t stride = (size_t)gridDim.x * blockDim.x;
+    for (size_t e = (size_t)blockIdx.x * blockDim.x + threadIdx.x; e < nbins; e += stride) {
+        const unsigned long long *w = bins + WORDS * e;
+        unsigned long long h, l;
+        if (WORDS == kWideWords) {
+            l = w[1];
+            h = w[3];
+            add_u128(h, l, w[2] >> 32, w[2] << 32);
+            h += w[4] << 32;
+        } else {
+            h = w[1];
+            l = w[2];
+        }
+        f[e] = __dadd_rn((double)h, __dmul_rn((double)l, 1.0 / 18446744073709551616.0));
+        c[e] = w[0];
+    }
 }
 
 // Local escaped distributions (calc_escaped_distributions, diagnostics.f90:
@@ -1115,13 +1226,14 @@ __global__ void __launch_bounds__(256) local_dist_kernel(const DevParticles P, i
 // fz(nmu, npb, nrx, nry, 2), low face first; a face whose array the
 // reference does not allocate (y below 2D, z below 3D) is skipped.
 __global__ void __launch_bounds__(256) local_escaped_kernel(const DevParticles P, int64_t n,
-                                                            const LocalDistArgs a,
+                                                            const LocalBins g,
                                                             unsigned long long *fx,
                                                             unsigned long long *fy,
                                                             unsigned long long *fz) {
+    const LocalDistArgs &a = g.a;
     const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
-    const LocalBin b = local_bin(P, i, a);
+    const LocalBin b = local_bin(P, i, g);
     if (!(b.ip > 0 && b.ip < a.npb) || b.imu < 1 || b.imu > a.nmu) return;
     const bool cx = b.ix >= 1 && b.ix <= a.nrx, cy = b.iy >= 1 && b.iy <= a.nry;
     const bool cz = b.iz >= 1 && b.iz <= a.nrz;
@@ -1146,85 +1258,46 @@ __global__ void __launch_bounds__(256) local_escaped_kernel(const DevParticles P
     }
 }
 
-// Global distribution with pitch-angle bins (calc_particle_distributions
-// :773-779, calc_escaped_distributions :949-957): fglobal(nmu, npp) or, with
-// by_face, fescaped(nmu, npp, |count_flag|); the particle's own weight.
-// p == pmax and mu == 1 index past the last bin in the reference and are
-// dropped.
-__device__ __forceinline__ int64_t mu_bin(const DevParticles &P, int64_t i, const MuDistArgs &a) {
-    const double p = P.p[i], mu = P.mu[i];
-    if (!(p > a.pmin && p <= a.pmax && mu >= -1.0 && mu <= 1.0)) return -1;
-    const int ip = (int)floor((log10(p) - a.pmin_log) / a.dp_log) + 1;
-    const int imu = (int)floor((mu + 1.0) / a.dmu) + 1;
-    if (ip < 1 || ip > a.npp || imu < 1 || imu > a.nmu) return -1;
-    int64_t face = 0;
-    if (a.by_face) {
-        const int flag = P.count_flag[i];
-        if (flag >= 0 || flag < -6) return -1;
-        face = -flag - 1;
-    }
-    return (int64_t)(imu - 1) + (int64_t)a.nmu * ((int64_t)(ip - 1) + (int64_t)a.npp * face);
-}
-
+// More bins than shared memory takes: one particle per thread.
 __global__ void __launch_bounds__(256) mu_dist_kernel(const DevParticles P, int64_t n,
-                                                      const MuDistArgs a,
+                                                      const MuBins g,
                                                       unsigned long long *bins) {
     const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
-    const int64_t b = mu_bin(P, i, a);
+    const int64_t b = mu_bin(P, i, g);
     if (b >= 0) bin_add(bins, (size_t)b, P.weight[i]);
 }
 
-// The same with block-private bins in shared memory (nbins triples) and
-// lanes of a warp that share a bin merged first, as histogram_kernel does.
-__global__ void __launch_bounds__(256) mu_dist_shared_kernel(const DevParticles P, int64_t n,
-                                                             const MuDistArgs a, int nbins,
-                                                             unsigned long long *bins) {
-    extern __shared__ unsigned long long sh[];
-    for (int b = threadIdx.x; b < 3 * nbins; b += blockDim.x) sh[b] = 0ull;
-    __syncthreads();
-    const int64_t stride = (int64_t)gridDim.x * blockDim.x;
-    const int64_t start = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    const int64_t iters = (n + stride - 1) / stride;
-    for (int64_t it = 0; it < iters; ++it) {
-        const int64_t i = start + it * stride;
-        int bin = -1;
-        unsigned long long wh = 0, wl = 0;
-        if (i < n) {
-            bin = (int)mu_bin(P, i, a);
-            if (bin >= 0) fixed_split(P.weight[i], wh, wl);
-        }
-        const unsigned grp = __match_any_sync(0xffffffffu, bin);
-        const int leader = __ffs(grp) - 1;
-        unsigned long long sh_h = 0, sh_l = 0;
-        unsigned m = grp;
-        while (m) {
-            const int src = __ffs(m) - 1;
-            m &= m - 1;
-            const unsigned long long oh = __shfl_sync(grp, wh, src);
-            const unsigned long long ol = __shfl_sync(grp, wl, src);
-            add_u128(sh_h, sh_l, oh, ol);
-        }
-        if (bin >= 0 && (int)(threadIdx.x & 31) == leader) {
-            atomicAdd(&sh[3 * bin], (unsigned long long)__popc(grp));
-            atomic_add_u128(&sh[3 * bin + 1], &sh[3 * bin + 2], sh_h, sh_l);
-        }
-    }
-    __syncthreads();
-    for (int b = threadIdx.x; b < nbins; b += blockDim.x) {
-        if (sh[3 * b]) atomicAdd(&bins[3 * b], sh[3 * b]);
-        atomic_add_u128(&bins[3 * b + 1], &bins[3 * b + 2], sh[3 * b + 1], sh[3 * b + 2]);
-    }
-}
+// Shared memory of bins_shared_kernel: a table of up to 2048 bins, 72 KiB, at
+// least three blocks of which fit an SM; up to 6144 bins, 216 KiB, one block.
+constexpr int kSharedBins = 6144;
 
-// Largest table the shared-memory path holds: 8192 triples, 192 KiB.
-constexpr int kMuSharedBins = 8192;
+// A local distribution of up to this many elements is summed in wide bins
+// (320 MiB).
+constexpr size_t kWideBins = (size_t)1 << 23;
+
+size_t local_dist_words(size_t nbins) {
+    return nbins * (nbins <= kWideBins ? (size_t)kWideWords : 3);
+}
 
 cudaError_t launch_local_dist(const DevParticles &P, int64_t n, const LocalDistArgs &a,
                               unsigned long long *bins, size_t nbins, cudaStream_t s) {
-    cudaError_t e = cudaMemsetAsync(bins, 0, sizeof(unsigned long long) * 3 * nbins, s);
+    cudaError_t e = cudaMemsetAsync(bins, 0, sizeof(unsigned long long) * local_dist_words(nbins), s);
     if (e != cudaSuccess || n <= 0) return e;
-    local_dist_kernel<<<(unsigned)((n + 255) / 256), 256, 0, s>>>(P, n, a, bins);
+    const unsigned blocks = (unsigned)((n + 255) / 256);
+    const LocalBins g = make_local_bins(a);
+    if (nbins <= kWideBins) local_dist_kernel<true><<<blocks, 256, 0, s>>>(P, n, g, bins);
+    else local_dist_kernel<false><<<blocks, 256, 0, s>>>(P, n, g, bins);
+    return cudaGetLastError();
+}
+
+cudaError_t launch_bins_out(const unsigned long long *bins, size_t nbins, int words, double *f,
+                            unsigned long long *c, cudaStream_t s) {
+    if (nbins == 0) return cudaSuccess;
+    const size_t want = (nbins + 255) / 256;
+    const unsigned blocks = (unsigned)(want < 65535 ? want : 65535);
+    if (words == kWideWords) bins_out_kernel<kWideWords><<<blocks, 256, 0, s>>>(bins, nbins, f, c);
+    else bins_out_kernel<3><<<blocks, 256, 0, s>>>(bins, nbins, f, c);
     return cudaGetLastError();
 }
 
@@ -1232,7 +1305,8 @@ cudaError_t launch_local_escaped(const DevParticles &P, int64_t n, const LocalDi
                                  unsigned long long *fx, unsigned long long *fy,
                                  unsigned long long *fz, cudaStream_t s) {
     if (n <= 0) return cudaSuccess;
-    local_escaped_kernel<<<(unsigned)((n + 255) / 256), 256, 0, s>>>(P, n, a, fx, fy, fz);
+    local_escaped_kernel<<<(unsigned)((n + 255) / 256), 256, 0, s>>>(P, n, make_local_bins(a), fx, fy,
+                                                                      fz);
     return cudaGetLastError();
 }
 
@@ -1240,17 +1314,21 @@ cudaError_t launch_mu_dist(const DevParticles &P, int64_t n, const MuDistArgs &a
                            unsigned long long *bins, size_t nbins, cudaStream_t s) {
     cudaError_t e = cudaMemsetAsync(bins, 0, sizeof(unsigned long long) * 3 * nbins, s);
     if (e != cudaSuccess || n <= 0) return e;
-    if (nbins <= (size_t)kMuSharedBins) {
-        const size_t shmem = sizeof(unsigned long long) * 3 * nbins;
+    const MuBins g{a, make_log_bins(a.pmin_log, a.dp_log), make_even_bins(-1.0, a.dmu)};
+    if (nbins <= (size_t)kSharedBins) {
+        const size_t shmem = sizeof(unsigned int) * kBinWords * nbins;
         // per device, so set on every call (it is cheap)
-        e = cudaFuncSetAttribute(mu_dist_shared_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 (int)(sizeof(unsigned long long) * 3 * kMuSharedBins));
+        e = cudaFuncSetAttribute(bins_shared_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                 (int)(sizeof(unsigned int) * kBinWords * kSharedBins));
         if (e != cudaSuccess) return e;
+        // Every block adds its table to the global one: four blocks per SM as
+        // far as they fit, fewer where a table costs more than its particles.
         int64_t blocks = (n + 255) / 256;
-        if (blocks > 1024) blocks = 1024;
-        mu_dist_shared_kernel<<<(unsigned)blocks, 256, shmem, s>>>(P, n, a, (int)nbins, bins);
+        const int64_t most = std::max<int64_t>(152, std::min<int64_t>(608, n / (4 * (int64_t)nbins)));
+        if (blocks > most) blocks = most;
+        bins_shared_kernel<<<(unsigned)blocks, 256, shmem, s>>>(P, n, g, (int)nbins, bins);
     } else {
-        mu_dist_kernel<<<(unsigned)((n + 255) / 256), 256, 0, s>>>(P, n, a, bins);
+        mu_dist_kernel<<<(unsigned)((n + 255) / 256), 256, 0, s>>>(P, n, g, bins);
     }
     return cudaGetLastError();
 }
@@ -1258,7 +1336,7 @@ cudaError_t launch_mu_dist(const DevParticles &P, int64_t n, const MuDistArgs &a
 cudaError_t launch_quick_check(const DevParticles &P, int64_t n, DevCounters *cnt, cudaStream_t s) {
     if (n <= 0) return cudaSuccess;
     int64_t blocks = (n + 255) / 256;
-    if (blocks > 2048) blocks = 2048;
+    if (blocks > 608) blocks = 608;
     quick_check_kernel<<<(unsigned)blocks, 256, 0, s>>>(P, n, cnt);
     return cudaGetLastError();
 }
