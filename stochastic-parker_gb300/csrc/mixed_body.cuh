@@ -160,56 +160,58 @@ __device__ __forceinline__ bool interp_global(const MixedRunArgs &a, const Pos &
 // interp_global for a whole warp, each lane's particle by a group of lanes:
 // lane j of a group of 2 (2D) or 4 (3D) reads the 32-byte sector j of a
 // corner's record for every particle of the group in turn, weighs and sums it,
-// and the sums change hands in shared memory.  A load instruction then touches
+// and the sums change hands.  A load instruction then touches
 // 16 (8) lines instead of 32 scattered sectors, and the L1 data pipe, which
 // spends a wavefront per line touched, delivers twice the records (random
 // records of 64 B: 2.3e11/s against 1.15e11; of 96 B: 1.96e11 against 9.9e10).
 // Weights and the order of the sums are interp_global's.  want: the lane's
 // particle makes a push.  All lanes of the warp call; buf: its kGatherBuf<NDIM>
 // floats.  False where the position is outside the ghost range.
-// The buffer holds planes of one 16-byte chunk per lane: plane j + sectors h is
+// 3D's buffer holds planes of one 16-byte chunk per lane: plane j + sectors h is
 // half h of sector j, rotated by j lanes, so that neither the writes of a
-// group's sectors nor the reads of a plane share banks.  In 3D the last plane
-// keeps one float per lane, the 21st value.
+// group's sectors nor the reads of a plane share banks; the last plane keeps one
+// float per lane, the 21st value.  2D exchanges its sums by shuffles.
 constexpr int kGatherPlane = 4 * 32;
-template <int NDIM>
-constexpr int kGatherBuf = NDIM == 2 ? 4 * kGatherPlane : 5 * kGatherPlane + 32;
+// s += w * the 8 floats at r (32-byte aligned).
+__device__ __forceinline__ void add_sector(const float *r, float w, float (&s)[8]) {
+    float g[8];
+    ld8(r, g);
+#pragma unroll
+    for (int e = 0; e < 8; ++e) s[e] = fmaf(g[e], w, s[e]);
+}
 
-template <int NDIM, int NV>
-__device__ __forceinline__ bool interp_group(const MixedRunArgs &a, const Pos &q, float rt,
-                                             bool want, float *buf, float f[NV]) {
+// 2D: no branch around the loads, so that both members' are in flight at once
+// (43.7 -> 41.5 ms for 2e6 particles); a member without a push stands for cell
+// 0, whose sums nobody reads.  3D, where a quarter of the members of a late
+// chunk have none and a group's fourth lane has no sector: skipped (24.8 against
+// 26.6 ms for 1e6 particles).
+template <int NDIM>
+constexpr uint32_t kNoCell = NDIM == 2 ? 0u : 0xffffffffu;
+template <int NDIM>
+constexpr int kGatherBuf = NDIM == 2 ? 1 : 5 * kGatherPlane + 32;
+
+// TWO: both frames.  A template argument, because a branch around a load of the
+// second frame keeps the loads that follow from being issued with it.
+template <int NDIM, int NV, bool TWO>
+__device__ __forceinline__ void group_sums(const MixedRunArgs &a, const Pos &q, float rt,
+                                           uint32_t mine, float *buf, float f[NV]) {
     constexpr int R = (NDIM == 2) ? kRec2D : kRec3D;
     constexpr int G = (NDIM == 2) ? 2 : 4, kSectors = (NDIM == 2) ? 2 : 3;
     constexpr int kCorners = (NDIM == 2) ? 4 : 8;
     const int lane = threadIdx.x & 31, sub = lane & (G - 1);
-    const int ix = q.cx + 2, iy = q.cy + 2, iz = (NDIM == 3) ? q.cz + 2 : 0;
-    bool ok = want;
-    if (want && ((unsigned)ix > (unsigned)(a.nxg - 2) || (unsigned)iy > (unsigned)(a.nyg - 2) ||
-                 (NDIM == 3 && (unsigned)iz > (unsigned)(a.nzg - 2)))) {
-        record_guard(a.cnt, ix, iy, iz, 1);
-        ok = false;
-    }
     const size_t row = (size_t)a.nxg, plane = (size_t)a.nxg * a.nyg;
-    // 2D: no branch around the loads, so that both members' are in flight at
-    // once (46.9 -> 41.5 ms for 2e6 particles); a member without a push stands
-    // for cell 0, whose sums nobody reads.  3D, where a quarter of the members
-    // of a late chunk have none and a group's fourth lane has no sector: skipped
-    // (24.8 against 26.6 ms for 1e6 particles).
-    const uint32_t none = NDIM == 2 ? 0u : 0xffffffffu;
-    const uint32_t mine = ok ? (uint32_t)ix + (uint32_t)a.nxg * ((uint32_t)iy +
-                                                                  (uint32_t)a.nyg * (uint32_t)iz)
-                             : none;
     const float *rec1 = a.rec1 + 8 * sub, *rec2 = a.rec2 + 8 * sub;
-    __syncwarp();   // the group has read its last sums
+    float sums[NDIM == 2 ? 2 : 1][8];   // 2D: of both members
+    if (NDIM == 3) __syncwarp();   // the group has read its last sums
 #pragma unroll
     for (int m = 0; m < G; ++m) {
         const uint32_t base = __shfl_sync(0xffffffffu, mine, m, G);
         const float fx = __shfl_sync(0xffffffffu, q.fx, m, G);
         const float fy = __shfl_sync(0xffffffffu, q.fy, m, G);
         const float fz = (NDIM == 3) ? __shfl_sync(0xffffffffu, q.fz, m, G) : 0.0f;
-        const float tm = a.time_interp ? __shfl_sync(0xffffffffu, rt, m, G) : 0.0f;
-        if (NDIM == 3 && (base == none || sub >= kSectors)) continue;
-        float s[8];
+        const float tm = TWO ? __shfl_sync(0xffffffffu, rt, m, G) : 0.0f;
+        if (NDIM == 3 && (base == kNoCell<NDIM> || sub >= kSectors)) continue;
+        float (&s)[8] = sums[NDIM == 2 ? m : 0];
 #pragma unroll
         for (int e = 0; e < 8; ++e) s[e] = 0.0f;
         const float *r1 = rec1 + (size_t)R * base;
@@ -219,19 +221,11 @@ __device__ __forceinline__ bool interp_group(const MixedRunArgs &a, const Pos &q
             float wc = ((c & 1) ? fx : 1.0f - fx) * ((c & 2) ? fy : 1.0f - fy);
             if (NDIM == 3) wc *= ((c & 4) ? fz : 1.0f - fz);
             const size_t off = R * ((c & 1) + ((c & 2) ? row : 0) + ((c & 4) ? plane : 0));
-            float w1 = wc;
-            if (a.time_interp) w1 = wc * (1.0f - tm);
-            float g[8];
-            ld8(r1 + off, g);
-#pragma unroll
-            for (int e = 0; e < 8; ++e) s[e] = fmaf(g[e], w1, s[e]);
-            if (a.time_interp) {
-                const float w2 = wc * tm;
-                ld8(r2 + off, g);
-#pragma unroll
-                for (int e = 0; e < 8; ++e) s[e] = fmaf(g[e], w2, s[e]);
-            }
+            const float w1 = TWO ? wc * (1.0f - tm) : wc;
+            add_sector(r1 + off, w1, s);
+            if (TWO) add_sector(r2 + off, wc * tm, s);
         }
+        if (NDIM == 2) continue;
         const int who = lane - sub + m;
         float *to = buf + kGatherPlane * sub + 4 * ((who + sub) & 31);
         *reinterpret_cast<float4 *>(to) = make_float4(s[0], s[1], s[2], s[3]);
@@ -240,6 +234,18 @@ __device__ __forceinline__ bool interp_group(const MixedRunArgs &a, const Pos &q
         else
             *reinterpret_cast<float4 *>(to + kGatherPlane * kSectors) =
                 make_float4(s[4], s[5], s[6], s[7]);
+    }
+    if (NDIM == 2) {
+        // Each lane of the pair keeps its own particle's half and gets the other
+        // (8 shuffles and selects; through shared memory 44.4 against 39.5 ms).
+        constexpr int kOdd = NDIM == 2 ? 1 : 0;
+#pragma unroll
+        for (int e = 0; e < 8; ++e) {
+            const float got = __shfl_xor_sync(0xffffffffu, sub ? sums[0][e] : sums[kOdd][e], 1);
+            f[e] = sub ? got : sums[0][e];
+            if (8 + e < NV) f[8 + e] = sub ? sums[kOdd][e] : got;
+        }
+        return;
     }
     __syncwarp();
 #pragma unroll
@@ -256,6 +262,23 @@ __device__ __forceinline__ bool interp_group(const MixedRunArgs &a, const Pos &q
         if (4 * v4 + 2 < NV) f[4 * v4 + 2] = g.z;
         if (4 * v4 + 3 < NV) f[4 * v4 + 3] = g.w;
     }
+}
+
+template <int NDIM, int NV>
+__device__ __forceinline__ bool interp_group(const MixedRunArgs &a, const Pos &q, float rt,
+                                             bool want, float *buf, float f[NV]) {
+    const int ix = q.cx + 2, iy = q.cy + 2, iz = (NDIM == 3) ? q.cz + 2 : 0;
+    bool ok = want;
+    if (want && ((unsigned)ix > (unsigned)(a.nxg - 2) || (unsigned)iy > (unsigned)(a.nyg - 2) ||
+                 (NDIM == 3 && (unsigned)iz > (unsigned)(a.nzg - 2)))) {
+        record_guard(a.cnt, ix, iy, iz, 1);
+        ok = false;
+    }
+    const uint32_t mine = ok ? (uint32_t)ix + (uint32_t)a.nxg * ((uint32_t)iy +
+                                                                  (uint32_t)a.nyg * (uint32_t)iz)
+                             : kNoCell<NDIM>;
+    if (a.time_interp) group_sums<NDIM, NV, true>(a, q, rt, mine, buf, f);
+    else group_sums<NDIM, NV, false>(a, q, rt, mine, buf, f);
     return ok;
 }
 
@@ -730,31 +753,43 @@ __device__ __forceinline__ int next_nsp(int nsp, int interval) {
 // move_particle with the gathers of a whole warp (interp_group): the loop turns
 // once per push of the warp, ordinary and landing pushes through the same
 // code, until no lane's particle has one left before its pause or the end of
-// the interval.  All lanes call; valid: the lane has a particle.
+// the interval.  All lanes call; i, valid: the lane's particle; paused: it has
+// pushes left.  (Lanes that take another particle when theirs is done, as the
+// FP64 mover's do, lose more in shared records than they gain: 3D 29.8 against
+// 24.3 ms for 1e6 particles, 2D 43.8 against 39.3 for 2e6.)
 template <int NDIM, bool NLGC>
 __device__ __forceinline__ uint32_t move_warp(const MixedRunArgs &a, const MixedConsts &k,
                                               const DevParticles &P, int64_t i, bool valid,
-                                              bool &active, uint32_t limit, float *buf) {
+                                              bool &paused, uint32_t limit, float *buf) {
     constexpr int NV = (NDIM == 2) ? 15 : 21;
     uint32_t pushes = 0;
-    active = false;
+    paused = false;
     double x_in = 0.0, y_in = 0.0, z_in = 0.0, p_in = 0.0, t_in = 0.0;
-    const double *wp = P.weight + i;
-    Pos q = {0, 0, 0, 0.0f, 0.0f, 0.0f};
+    Pos q = {0, 0, 0, 0.0f, 0.0f, 0.0f}, q_in = q;
     float p_f0 = 0.0f, tau_f0 = 0.0f, dt = 0.0f, mu = 0.0f;
-    double target_d = 0.0;
+    double target_d = 0.0, landed_d = 0.0;
     float target = 0.0f;                   // (float)target_d
     int flag = 0, nsp = 0;
     uint32_t ctr = 0, ti = 0, ts = 0;
+    float z2 = 0.0f;                       // 2D out-of-plane drift, physical units
+    float p = 0.0f, pc = 0.0f, tau = 0.0f, tc = 0.0f, dtr = 0.0f;
+    bool landed = false;                   // on the target: written as t0 + landed_d
+    float uX = 0.0f, uY = 0.0f, uZ = 0.0f, uP = 0.0f;
+    // alive: in the box, with fine-step targets left in the interval
+    bool alive = false;
+
     if (valid) {
         x_in = P.x[i]; y_in = P.y[i]; z_in = P.z[i];
         p_in = P.p[i]; t_in = P.t[i];
         cell_of(x_in, a.xmin, a.dx, q.cx, q.fx);
         cell_of(y_in, a.ymin, a.dy, q.cy, q.fy);
         if (NDIM == 3) cell_of(z_in, a.zmin, a.dz, q.cz, q.fz);
+        q_in = q;
         p_f0 = (float)p_in;
+        p = p_f0;
         const double tau_in = t_in - a.t0;
         tau_f0 = (float)tau_in;
+        tau = tau_f0;
         dt = (float)P.dt[i];
         flag = P.count_flag[i];
         nsp = P.nsteps_pushed[i];
@@ -765,32 +800,20 @@ __device__ __forceinline__ uint32_t move_warp(const MixedRunArgs &a, const Mixed
         const double stepd = ceil(tau_in / a.dt_fine);
         target_d = (stepd <= 0.0) ? a.dt_fine : stepd * a.dt_fine;
         if (target_d > a.dtf) target_d = a.dtf;
-    }
-    const Pos q_in = q;
-    float z2 = 0.0f;                       // 2D out-of-plane drift, physical units
-    float p = p_f0, pc = 0.0f;
-    float tau = tau_f0, tc = 0.0f;
-    float landed_at = -1.0f;               // landed on the target, written as t0 + target_d
-    double landed_d = 0.0;
-    float uX = 0.0f, uY = 0.0f, uZ = 0.0f, uP = 0.0f;
-    if (valid) {
+        target = (float)target_d;
         if (p < 0.0f && flag == 1) {
             flag = 0;
-            atomic_add_fixed(&a.cnt->negp_hi, &a.cnt->negp_lo, *wp);
+            atomic_add_fixed(&a.cnt->negp_hi, &a.cnt->negp_lo, P.weight[i]);
         } else {
-            boundary<NDIM>(a, k, q, true, flag, wp);
+            boundary<NDIM>(a, k, q, true, flag, P.weight + i);
         }
+        alive = flag == 1 && target_d < a.limit;
     }
-    // alive: in the box, with fine-step targets left in the interval
-    bool alive = valid && flag == 1 && target_d < a.limit;
-    target = (float)target_d;
-    bool paused = false;
-    float dtr = 0.0f;
     for (;;) {
         bool want = false, fixed = false;
         while (alive && flag == 1) {
             if (tau - tc < target) {
-                negp_or_boundary<NDIM>(a, k, q, p - pc, flag, wp);
+                negp_or_boundary<NDIM>(a, k, q, p - pc, flag, P.weight + i);
                 if (flag != 1) break;
                 if (limit != 0 && pushes >= limit) {
                     paused = true;   // between pushes: the next launch resumes from t
@@ -817,9 +840,9 @@ __device__ __forceinline__ uint32_t move_warp(const MixedRunArgs &a, const Mixed
                     fixed = true;
                     break;
                 }
-                negp_or_boundary<NDIM>(a, k, q, p - pc, flag, wp);
+                negp_or_boundary<NDIM>(a, k, q, p - pc, flag, P.weight + i);
             } else if (tau - tc == target) {
-                landed_at = 1.0f;      // reached the target without overshoot
+                landed = true;         // reached the target without overshoot
                 landed_d = target_d;
             }
             target_d = target_d + a.dt_fine;
@@ -856,14 +879,14 @@ __device__ __forceinline__ uint32_t move_warp(const MixedRunArgs &a, const Mixed
             nsp = next_nsp(nsp, a.nsteps_interval);
             if (fix) {
                 tau = target; tc = 0.0f;
-                landed_at = 1.0f;
+                landed = true;
                 landed_d = target_d;
-                negp_or_boundary<NDIM>(a, k, q, p - pc, flag, wp);
+                negp_or_boundary<NDIM>(a, k, q, p - pc, flag, P.weight + i);
                 target_d = target_d + a.dt_fine;
                 target = (float)target_d;
                 alive = target_d < a.limit;
             } else {
-                landed_at = -1.0f;
+                landed = false;
                 if (!(fabsf(tau) < 1e30f) || !(fabsf(p) < 1e30f) || !(q.fx <= 1.0f) ||
                     !(q.fy <= 1.0f) || !(q.fz <= 1.0f)) {
                     set_status(a.cnt, kStatusNonFinite);
@@ -879,8 +902,7 @@ __device__ __forceinline__ uint32_t move_warp(const MixedRunArgs &a, const Mixed
         else push_on(false);
     }
     if (!valid) return 0;
-    if (flag == 1 && !paused) boundary<NDIM>(a, k, q, false, flag, wp);
-    active = paused;
+    if (flag == 1 && !paused) boundary<NDIM>(a, k, q, false, flag, P.weight + i);
     // Write back input + change, computed in FP64.
     const double dcx = (double)(q.cx - q_in.cx) + ((double)q.fx - (double)q_in.fx);
     const double dcy = (double)(q.cy - q_in.cy) + ((double)q.fy - (double)q_in.fy);
@@ -893,13 +915,13 @@ __device__ __forceinline__ uint32_t move_warp(const MixedRunArgs &a, const Mixed
         P.z[i] = z_in + (double)z2;
     }
     P.p[i] = p_in + (((double)p - (double)pc) - (double)p_f0);
-    P.t[i] = landed_at >= 0.0f ? a.t0 + landed_d
-                               : t_in + (((double)tau - (double)tc) - (double)tau_f0);
+    P.t[i] = landed ? a.t0 + landed_d : t_in + (((double)tau - (double)tc) - (double)tau_f0);
     P.dt[i] = (double)dt;
     P.count_flag[i] = (int8_t)flag;
     P.nsteps_pushed[i] = nsp;
     P.nsteps_tracked[i] = 1;
     P.rng_ctr[i] = ctr;
+    if (a.pause) a.pause[i] = paused ? 1 : 0;
     return pushes;
 }
 

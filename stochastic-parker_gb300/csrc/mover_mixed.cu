@@ -61,11 +61,10 @@ __global__ void __launch_bounds__(128, NDIM == 2 ? GPAT_MIXED_MINB_2D : GPAT_MIX
                        const int64_t n) {
     __shared__ __align__(16) float gather[4][kGatherBuf<NDIM>];
     const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    bool active = false;
-    const uint32_t pushes = move_warp<NDIM, NLGC>(a, k, P, i, i < n, active, a.chunk_pushes,
+    bool paused;
+    const uint32_t pushes = move_warp<NDIM, NLGC>(a, k, P, i, i < n, paused, a.chunk_pushes,
                                                   gather[threadIdx.x >> 5]);
-    if (i < n && a.pause) a.pause[i] = active ? 1 : 0;
-    add_warp_counters(a.cnt, pushes, active, nullptr);
+    add_warp_counters(a.cnt, pushes, paused, nullptr);
 }
 
 // The global-gather chunk kernel with learned splitting: as a particle
@@ -84,12 +83,11 @@ __global__ void __launch_bounds__(128, NDIM == 2 ? GPAT_MIXED_MINB_2D : GPAT_MIX
     __syncthreads();
     __shared__ __align__(16) float gather[4][kGatherBuf<NDIM>];
     const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    bool active = false;
-    const uint32_t pushes = move_warp<NDIM, NLGC>(a, k, P, i, i < n, active, a.chunk_pushes,
+    bool paused;
+    const uint32_t pushes = move_warp<NDIM, NLGC>(a, k, P, i, i < n, paused, a.chunk_pushes,
                                                   gather[threadIdx.x >> 5]);
-    if (i < n && a.pause) a.pause[i] = active ? 1 : 0;
-    add_warp_counters(a.cnt, pushes, active, nullptr);
-    const bool fin = i < n && !active && P.count_flag[i] == 1;
+    add_warp_counters(a.cnt, pushes, paused, nullptr);
+    const bool fin = i < n && !paused && P.count_flag[i] == 1;
     if (!__any_sync(0xffffffffu, fin)) return;
     float h0[kMlpFeatures];
     if (fin) {
@@ -143,11 +141,11 @@ __global__ void __launch_bounds__(128, MINB)
             }
             const BatchRun &d = c_batch_runs[lo];
             const int64_t i = (t - tile_prefix[lo]) * 128 + threadIdx.x;
-            bool active = false;
+            bool paused;
             const uint32_t pushes =
-                move_warp<NDIM, NLGC>(d.a, d.k, d.P[parity], i, i < (int64_t)run_n[lo], active,
+                move_warp<NDIM, NLGC>(d.a, d.k, d.P[parity], i, i < (int64_t)run_n[lo], paused,
                                       d.a.chunk_pushes, gather[threadIdx.x >> 5]);
-            add_warp_counters(d.a.cnt, pushes, active, nactive_total);
+            add_warp_counters(d.a.cnt, pushes, paused, nactive_total);
         }
     }
 }
