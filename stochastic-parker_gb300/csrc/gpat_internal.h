@@ -252,6 +252,9 @@ cudaError_t launch_scatter_aux(const float *src, float *aux, int comp, size_t nc
                                cudaStream_t s);
 cudaError_t launch_fill(float *a, float v, size_t n, cudaStream_t s);
 cudaError_t launch_mover_fp64(const MoverArgs &a, int sm_count, cudaStream_t s);
+// The same in teams of kMoverTeam lanes, for launch_mover_fp64.
+constexpr int kMoverTeam = 8;
+cudaError_t launch_mover_fp64_team(const MoverArgs &a, int sm_count, cudaStream_t s);
 // Whether that launch orders n particles, for which MoverArgs::work has room
 // for kOrderHead + n words.
 constexpr int kOrderHead = 128;

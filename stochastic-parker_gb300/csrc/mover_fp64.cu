@@ -20,8 +20,16 @@
 #include "grid_common.cuh"
 #include "track_common.cuh"
 
+// Lanes that share one particle's interpolation: 1, or 8 in the translation unit
+// for calls with few particles (mover_fp64_team.cu).
+#ifndef GPAT_FP64_TEAM
+#define GPAT_FP64_TEAM 1
+#endif
+
 namespace gpat {
 namespace {
+
+constexpr int kTeam = GPAT_FP64_TEAM;
 
 // Packed record slots (fields.cu).
 enum R2 { A_VX, A_VY, A_BX, A_BY, A_BZ, A_DVXDX, A_DVYDY, A_DBXDX, A_DBXDY, A_DBYDX, A_DBYDY,
@@ -84,31 +92,8 @@ __device__ __forceinline__ void add_corner(const float *rec, double w, bool plai
     }
 }
 
-// NV variables of records of R floats interpolated with corner (ix, iy, iz)
-// and weights w, time-interpolated between the two frames; odd: per frame, a
-// value that needs the plain product (DevCounters::odd_fields, odd_aux).
-template <int NDIM, int NV, int R>
-__device__ __forceinline__ void interp_at(const MoverArgs &a, const float *rec1, const float *rec2,
-                                          const unsigned int *odd, const State &s, int ix, int iy,
-                                          int iz, const double *w, double f[NV]);
-
 // get_interp_paramters on the uniform grid: the lower corner (memory
 // indices) and the 8 weights; false outside the ghost cells.
-template <int NDIM>
-__device__ __forceinline__ bool uniform_cell(const MoverArgs &a, const State &s, int &ix, int &iy,
-                                             int &iz, double w[8]);
-
-// Interpolated fields at the particle: NV variables of records of R floats.
-template <int NDIM, int NV, int R>
-__device__ __forceinline__ bool interp(const MoverArgs &a, const float *rec1, const float *rec2,
-                                       const unsigned int *odd, const State &s, double f[NV]) {
-    int ix, iy, iz;
-    double w[8];
-    if (!uniform_cell<NDIM>(a, s, ix, iy, iz, w)) return false;
-    interp_at<NDIM, NV, R>(a, rec1, rec2, odd, s, ix, iy, iz, w, f);
-    return true;
-}
-
 template <int NDIM>
 __device__ __forceinline__ bool uniform_cell(const MoverArgs &a, const State &s, int &ix, int &iy,
                                              int &iz, double w[8]) {
@@ -123,10 +108,7 @@ __device__ __forceinline__ bool uniform_cell(const MoverArgs &a, const State &s,
     bool in = floor_next(px, fx, nextx) && fx >= -1 && fx <= nx;
     if (NDIM > 1) in = in && floor_next(py, fy, nexty) && fy >= -1 && fy <= ny;
     if (NDIM == 3) in = in && floor_next(pz, fz, nextz) && fz >= -1 && fz <= nz;
-    if (!in) {
-        set_status(a.cnt, kStatusIndexGuard);
-        return false;
-    }
+    if (!in) return false;
     const double rx = (px - nextx) + 1.0;
     const double ry = (NDIM > 1) ? (py - nexty) + 1.0 : 0.0;
     const double rz = (NDIM == 3) ? (pz - nextz) + 1.0 : 0.0;
@@ -145,6 +127,9 @@ __device__ __forceinline__ bool uniform_cell(const MoverArgs &a, const State &s,
     return true;
 }
 
+// NV variables of records of R floats interpolated with corner (ix, iy, iz)
+// and weights w, time-interpolated between the two frames; odd: per frame, a
+// value that needs the plain product (DevCounters::odd_fields, odd_aux).
 template <int NDIM, int NV, int R>
 __device__ __forceinline__ void interp_at(const MoverArgs &a, const float *rec1, const float *rec2,
                                           const unsigned int *odd, const State &s, int ix, int iy,
@@ -178,6 +163,77 @@ __device__ __forceinline__ void interp_at(const MoverArgs &a, const float *rec1,
 #pragma unroll
         for (int v = 0; v < NV; ++v) f[v] = f[v] * rt1 + f2[v] * rt;
     }
+}
+
+// interp_at by the kTeam lanes of a team for the particle of its first lane: lane
+// j sums variables j, j + kTeam, ...  The FP64 pipe takes as long for one lane as
+// for 32, so with few particles the other lanes' share comes for nothing.  All
+// lanes of the warp call; want: the first lane's particle makes a push.
+template <int NDIM, int NV, int R>
+__device__ __forceinline__ void interp_team(const MoverArgs &a, const float *rec1,
+                                            const float *rec2, const unsigned int *odd,
+                                            const State &s, bool want, int ix, int iy, int iz,
+                                            const double *w, double f[NV]) {
+    constexpr int kCorners = NDIM == 3 ? 8 : NDIM == 2 ? 4 : 2;
+    constexpr int K = (NV + kTeam - 1) / kTeam;
+    static_assert(K * kTeam <= R, "a lane's last variable lies inside the record");
+    const unsigned all = 0xffffffffu;
+    const int sub = threadIdx.x & (kTeam - 1);
+    uint32_t cell = want ? (uint32_t)ix + (uint32_t)a.nxg * ((uint32_t)iy +
+                                                             (uint32_t)a.nyg * (uint32_t)iz)
+                         : 0u;
+    cell = __shfl_sync(all, cell, 0, kTeam);
+    double wc[kCorners];
+#pragma unroll
+    for (int c = 0; c < kCorners; ++c) wc[c] = __shfl_sync(all, want ? w[c] : 1.0, 0, kTeam);
+    double u[K], u2[K];
+#pragma unroll 1
+    for (int frame = a.time_interp ? 1 : 0; frame >= 0; --frame) {
+        const float *rec = (frame ? rec2 : rec1) + (size_t)R * cell + sub;
+        const bool plain = __ldg(odd + (a.time_interp ? frame : 0)) != 0u;
+#pragma unroll
+        for (int c = 0; c < kCorners; ++c) {
+            size_t off = (size_t)(c & 1);
+            if (c & 2) off += (size_t)a.nxg;
+            if (c & 4) off += (size_t)a.nxg * (size_t)a.nyg;
+            const Weight wt = weight(wc[c]);
+            float v[K];
+#pragma unroll
+            for (int k = 0; k < K; ++k) v[k] = __ldg(rec + (size_t)R * off + kTeam * k);
+            double pr[K];
+            // a branch of the whole warp: as a choice per lane both sides are computed
+            if (__any_sync(all, plain || !wt.ok)) {
+#pragma unroll
+                for (int k = 0; k < K; ++k) pr[k] = 0.0 + (double)v[k] * wc[c];
+            } else {
+#pragma unroll
+                for (int k = 0; k < K; ++k) pr[k] = k & 1 ? widen(v[k]) * wc[c] : scaled(v[k], wt);
+            }
+#pragma unroll
+            for (int k = 0; k < K; ++k) u[k] = c == 0 ? pr[k] : u[k] + pr[k];
+        }
+        if (frame) {
+#pragma unroll
+            for (int k = 0; k < K; ++k) u2[k] = u[k];
+        }
+    }
+    if (a.time_interp) {
+        const double rt = __shfl_sync(all, div_by(s.t - a.t0, a.dtf, a.rdtf), 0, kTeam);
+        const double rt1 = 1.0 - rt;
+#pragma unroll
+        for (int k = 0; k < K; ++k) u[k] = u[k] * rt1 + u2[k] * rt;
+    }
+#pragma unroll
+    for (int v = 0; v < NV; ++v) f[v] = __shfl_sync(all, u[v / kTeam], v % kTeam, kTeam);
+}
+
+template <int NDIM, int NV, int R>
+__device__ __forceinline__ void interpolate(const MoverArgs &a, const float *rec1,
+                                            const float *rec2, const unsigned int *odd,
+                                            const State &s, bool want, int ix, int iy, int iz,
+                                            const double *w, double f[NV]) {
+    if (kTeam > 1) interp_team<NDIM, NV, R>(a, rec1, rec2, odd, s, want, ix, iy, iz, w, f);
+    else if (want) interp_at<NDIM, NV, R>(a, rec1, rec2, odd, s, ix, iy, iz, w, f);
 }
 
 // Field values at the particle under the reference's names.
@@ -1433,65 +1489,55 @@ __device__ __forceinline__ void run_push(const MoverArgs &a, State &s, const Fld
     }
 }
 
+// One push of the particles of the lanes that want one; false where it could
+// not be made.  In teams all lanes of the warp call (interpolate).
 template <int NDIM, bool FT, bool FULL, bool GRID, bool I3>
-__device__ __forceinline__ bool do_push(const MoverArgs &a, State &s, bool fixed_dt, Delta &d) {
+__device__ __forceinline__ bool do_push(const MoverArgs &a, State &s, bool want, bool fixed_dt,
+                                        Delta &d) {
+    // Spherical or non-uniform grid: corner and weights from the node
+    // positions (:1615-1630), all 32 variables.
+    GridCell c = {};
+    bool ok = want;
+    if (want) {
+        if (GRID)
+            ok = grid_cell(NDIM, a.spherical, a.xpos, a.nxg, a.ypos, a.nyg, a.zpos, a.nzg, s.x, s.y,
+                           s.z, c);
+        else
+            ok = uniform_cell<NDIM>(a, s, c.ix, c.iy, c.iz, c.w);
+        if (!ok) set_status(a.cnt, kStatusIndexGuard);
+    }
     Fld f;
     double av[16];
     const double *aux = nullptr;
-    if (GRID) {
-        // Spherical or non-uniform grid: corner and weights from the node
-        // positions (:1615-1630), all 32 variables.
-        GridCell c;
-        if (!grid_cell(NDIM, a.spherical, a.xpos, a.nxg, a.ypos, a.nyg, a.zpos, a.nzg, s.x, s.y,
-                       s.z, c)) {
-            set_status(a.cnt, kStatusIndexGuard);
-            return false;
-        }
+    if (FULL || GRID) {
         double v[32];
-        interp_at<NDIM, 32, 32>(a, a.full1, a.full2, a.cnt->odd_fields, s, c.ix, c.iy, c.iz, c.w, v);
+        interpolate<NDIM, 32, 32>(a, a.full1, a.full2, a.cnt->odd_fields, s, ok, c.ix, c.iy, c.iz,
+                                  c.w, v);
         f = named_full(v);
-        if (NDIM == 3 && a.surf_on) surface_heights(a, s, c.ix, c.iy, c.iz, c.w);
         if (a.aux1 && (a.deltab_flag || a.correlation_flag)) {
-            interp_at<NDIM, 16, 16>(a, a.aux1, a.aux2, a.cnt->odd_aux, s, c.ix, c.iy, c.iz, c.w, av);
-            aux = av;
-        }
-        Geo geo = {a.dx, a.dy, a.dz};
-        if (a.nonuniform) {
-            // the pushes' own search (no offset shift): X[k] - X[k - 1]
-            geo.dxm = __ldg(a.xpos + c.kx) - __ldg(a.xpos + c.kx - 1);
-            if (NDIM > 1) geo.dym = __ldg(a.ypos + c.ky) - __ldg(a.ypos + c.ky - 1);
-            if (NDIM == 3) geo.dzm = __ldg(a.zpos + c.kz) - __ldg(a.zpos + c.kz - 1);
-        }
-        if (a.spherical) run_push<NDIM, FT, true, I3>(a, s, f, aux, geo, fixed_dt, d);
-        else run_push<NDIM, FT, false, I3>(a, s, f, aux, geo, fixed_dt, d);
-        if (!finite_bits(s.x) || !finite_bits(s.y) || !finite_bits(s.z) || !finite_bits(s.p) ||
-            !finite_bits(s.t) || (FT && (!finite_bits(s.v) || !finite_bits(s.mu)))) {
-            set_status(a.cnt, kStatusNonFinite);
-            return false;
-        }
-        return true;
-    }
-    if (FULL) {
-        double v[32];
-        int ix, iy, iz;
-        double w[8];
-        if (!uniform_cell<NDIM>(a, s, ix, iy, iz, w)) return false;
-        interp_at<NDIM, 32, 32>(a, a.full1, a.full2, a.cnt->odd_fields, s, ix, iy, iz, w, v);
-        f = named_full(v);
-        if (NDIM == 3 && a.surf_on) surface_heights(a, s, ix, iy, iz, w);
-        if (a.aux1 && (a.deltab_flag || a.correlation_flag)) {
-            if (!interp<NDIM, 16, 16>(a, a.aux1, a.aux2, a.cnt->odd_aux, s, av)) return false;
+            interpolate<NDIM, 16, 16>(a, a.aux1, a.aux2, a.cnt->odd_aux, s, ok, c.ix, c.iy, c.iz,
+                                      c.w, av);
             aux = av;
         }
     } else {
         constexpr int NV = (NDIM == 2) ? 15 : 21;
         constexpr int R = (NDIM == 2) ? kRec2D : kRec3D;
         double v[NV];
-        if (!interp<NDIM, NV, R>(a, a.rec1, a.rec2, a.cnt->odd_fields, s, v)) return false;
+        interpolate<NDIM, NV, R>(a, a.rec1, a.rec2, a.cnt->odd_fields, s, ok, c.ix, c.iy, c.iz, c.w,
+                                 v);
         f = named_packed<NDIM>(v);
     }
-    const Geo geo = {a.dx, a.dy, a.dz};
-    run_push<NDIM, FT, false, I3>(a, s, f, aux, geo, fixed_dt, d);
+    if (!ok) return false;
+    if ((FULL || GRID) && NDIM == 3 && a.surf_on) surface_heights(a, s, c.ix, c.iy, c.iz, c.w);
+    Geo geo = {a.dx, a.dy, a.dz};
+    if (GRID && a.nonuniform) {
+        // the pushes' own search (no offset shift): X[k] - X[k - 1]
+        geo.dxm = __ldg(a.xpos + c.kx) - __ldg(a.xpos + c.kx - 1);
+        if (NDIM > 1) geo.dym = __ldg(a.ypos + c.ky) - __ldg(a.ypos + c.ky - 1);
+        if (NDIM == 3) geo.dzm = __ldg(a.zpos + c.kz) - __ldg(a.zpos + c.kz - 1);
+    }
+    if (GRID && a.spherical) run_push<NDIM, FT, true, I3>(a, s, f, aux, geo, fixed_dt, d);
+    else run_push<NDIM, FT, false, I3>(a, s, f, aux, geo, fixed_dt, d);
     if (!finite_bits(s.x) || !finite_bits(s.y) || !finite_bits(s.z) || !finite_bits(s.p) ||
         !finite_bits(s.t) || (FT && (!finite_bits(s.v) || !finite_bits(s.mu)))) {
         set_status(a.cnt, kStatusNonFinite);
@@ -1549,17 +1595,18 @@ __global__ void __launch_bounds__(128) mover_fp64_kernel(const MoverArgs a) {
     int32_t ntrk = 1;
     int trk_lo = 0, trk_hi = -1, trk_found = 0;
     bool have = false, more = true;
+    const bool taker = lane % kTeam == 0 && lane / kTeam < a.lanes;
     for (;;) {
         // Lanes without a particle take the next ones.
         while (more) {
-            const unsigned need = __ballot_sync(0xffffffffu, !have && lane < a.lanes);
+            const unsigned need = __ballot_sync(0xffffffffu, !have && taker);
             if (need == 0u) break;
             const int leader = __ffs(need) - 1;
             unsigned long long base = 0;
             if (lane == leader) base = atomicAdd(&a.cnt->next, (unsigned long long)__popc(need));
             base = __shfl_sync(0xffffffffu, base, leader);
             more = (int64_t)(base + __popc(need)) < a.n;
-            if (have || lane >= a.lanes) continue;
+            if (have || !taker) continue;
             i = (int64_t)(base + __popc(need & ((1u << lane) - 1u)));
             if (i >= a.n) continue;
             if (a.work) i = (int64_t)a.work[kOrderHead + i];
@@ -1632,8 +1679,10 @@ __global__ void __launch_bounds__(128) mover_fp64_kernel(const MoverArgs a) {
             }
             dt_target = dt_target + dt_fine;
         }
+        bool pushed = false;
+        if (kTeam > 1 || want) pushed = do_push<NDIM, FT, FULL, GRID, I3>(a, s, want, fixed, dl);
         if (want) {
-            if (do_push<NDIM, FT, FULL, GRID, I3>(a, s, fixed, dl)) {
+            if (pushed) {
                 ++pushes;
                 s.nsteps_pushed = (s.nsteps_pushed + 1) % a.nsteps_interval;
                 track_push<FT>(a, s, i, ntrk, trk_lo, trk_hi, trk_found);
@@ -1675,6 +1724,7 @@ __global__ void __launch_bounds__(128) mover_fp64_kernel(const MoverArgs a) {
     }
 }
 
+#if GPAT_FP64_TEAM == 1
 // ---------------------------------------------------------------------------
 // Work order.  A lane that takes a long particle last keeps its warp, and the
 // call, waiting; taken first, the others fill up around it.  The pushes left
@@ -1732,6 +1782,8 @@ __global__ void __launch_bounds__(256) order_scatter_kernel(const MoverArgs a, f
     if (i < a.n) a.work[kOrderHead + base[b] + rank] = (uint32_t)i;
 }
 
+#endif
+
 // Warps of a launch: one per SM sub-partition below five particles per lane of
 // that grid (97 280 on 152 SMs), two from there on.  A second warp fills the
 // gaps of the first (2D, 320 000 particles: 1.28e9 against 1.05e9 pushes/s; 3D
@@ -1742,19 +1794,34 @@ constexpr int kThreads = 128;
 
 }  // namespace
 
+#if GPAT_FP64_TEAM == 1
 bool mover_fp64_orders(int64_t n, int sm_count) { return n > (int64_t)sm_count * kThreads; }
 
 cudaError_t launch_mover_fp64(const MoverArgs &args, int sm_count, cudaStream_t s) {
     if (args.n <= 0) return cudaSuccess;
+    // Teams while every particle still gets one at once (2432 on 152 SMs): a push
+    // is then bound by its own chain of FP64 operations, and a team shortens it.
+    // An interval of 2432 particles in teams against 2500 without, ms: 2D shock 3.25
+    // against 3.88, 3D 6.2 against 8.9, 3D with two frames 7.0 against 12.6, focused
+    // transport 4.23 against 4.91, spherical 3D 0.78 against 1.09.  With more, teams
+    // would wait for one another.
+    if (args.n <= (int64_t)sm_count * kThreads / kMoverTeam)
+        return launch_mover_fp64_team(args, sm_count, s);
+#else
+static_assert(kTeam == kMoverTeam, "the rule of launch_mover_fp64");
+
+cudaError_t launch_mover_fp64_team(const MoverArgs &args, int sm_count, cudaStream_t s) {
+#endif
     MoverArgs a = args;
     const int threads = kThreads;
     // With fewer particles than lanes every warp takes a few.
     const int64_t one = (int64_t)sm_count * kThreads;
     const int64_t most = sm_count * (a.n >= 5 * one ? 2 : 1), warps = kThreads / 32;
     const int64_t blocks = std::min(most, (a.n + warps - 1) / warps);
-    a.lanes = (int)std::min<int64_t>(32, (a.n + warps * blocks - 1) / (warps * blocks));
+    a.lanes = (int)std::min<int64_t>(32 / kTeam, (a.n + warps * blocks - 1) / (warps * blocks));
     cudaError_t e = cudaMemsetAsync(&a.cnt->next, 0, sizeof(unsigned long long), s);
     if (e != cudaSuccess) return e;
+#if GPAT_FP64_TEAM == 1
     if (a.work) {
         e = cudaMemsetAsync(a.work, 0, sizeof(uint32_t) * kOrderHead, s);
         if (e != cudaSuccess) return e;
@@ -1766,6 +1833,7 @@ cudaError_t launch_mover_fp64(const MoverArgs &args, int sm_count, cudaStream_t 
         order_count_kernel<<<std::min(og, 8u * (unsigned)sm_count), 256, 0, s>>>(a, step0);
         order_scatter_kernel<<<og, 256, 0, s>>>(a, step0);
     }
+#endif
     const bool ft = a.focused_transport != 0;
     const bool full = ft || a.dpp_wave || a.dpp_shear || a.deltab_flag || a.correlation_flag ||
                       a.surf_on;

@@ -32,6 +32,7 @@ SOURCES = {
     "fields.cu": [],
     "particles.cu": ["-fmad=false"],   # injection draws match the oracle bit for bit
     "mover_fp64.cu": ["-fmad=false"],
+    "mover_fp64_team.cu": ["-fmad=false"],   # mover_fp64.cu for calls with few particles
     "mover_mixed.cu": [],
     "mover_tile.cu": [],
     "noalloc.cu": [],

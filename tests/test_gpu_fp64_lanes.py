@@ -1,7 +1,8 @@
 """The FP64 mover's work list and its integer forms, bit for bit against the
-oracle: fewer particles than warps, one more than the lanes of the small grid
-(taken in work order), enough for the large grid; cells of different sizes;
-fields with subnormal values and zeros."""
+oracle: fewer particles than warps, the most that are moved in teams of lanes
+and one more, one more than the lanes of the small grid (taken in work order),
+enough for the large grid; cells of different sizes; fields with subnormal
+values and zeros."""
 import numpy as np
 import pytest
 
@@ -54,7 +55,7 @@ def _frame2d(nx, ny, seed=3):
     return fields.planar_shock_2d(nx, ny, 0.0, 1.0, 0.0, 1.0, r=3.0, w=0.05, x0=0.5, db=db)
 
 
-@pytest.mark.parametrize("n", [1, 3, 700, 19457, 97281])
+@pytest.mark.parametrize("n", [1, 3, 700, 2432, 2433, 19457, 97281])
 def test_particle_counts_around_the_grids(n):
     _pair(2, n, _frame2d(32, 32))
 
