@@ -1579,7 +1579,7 @@ int gpat_particle_mover(gpat_handle_t *h, int focused_transport, int nlgc, doubl
                 L.count = h->learn_dev;
                 L.zsum = h->learn_dev + 1;
                 CK(cudaEventRecord(h->ev0, h->stream));
-                CK(launch_mover_learned(a, k, L, h->stream));
+                CK(launch_mover_learned(a, k, L, h->sm_count, h->stream));
                 CK(cudaEventRecord(h->ev1, h->stream));
                 CK(cudaMemcpyAsync(h->learn_host, h->learn_dev, 6 * sizeof(unsigned long long),
                                    cudaMemcpyDeviceToHost, h->stream));

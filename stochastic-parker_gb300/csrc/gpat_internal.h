@@ -264,7 +264,7 @@ cudaError_t launch_mover_mixed(const MoverArgs &a, const MixedConsts &c, int sm_
 MixedConsts make_mixed_consts(const MoverArgs &a);
 // The global-gather chunk launch with learned splitting of finished particles.
 cudaError_t launch_mover_learned(const MoverArgs &a, const MixedConsts &c, const FusedLearn &L,
-                                 cudaStream_t s);
+                                 int sm_count, cudaStream_t s);
 MixedRunArgs mixed_run_args(const MoverArgs &a);
 // Batched split-precision mover (see mover_mixed.cu).
 cudaError_t upload_batch_runs(const BatchRun *runs, int nruns, cudaStream_t s);

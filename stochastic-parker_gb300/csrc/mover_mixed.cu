@@ -55,14 +55,40 @@ MixedConsts make_mixed_consts(const MoverArgs &a) {
 
 namespace {
 
+// The particle of this lane where every spread-th lane has one.
+__device__ __forceinline__ int64_t spread_index(int spread, int64_t n, bool &valid) {
+    const int64_t at = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    const int64_t i = at >> (31 - __clz(spread));
+    valid = (at & (spread - 1)) == 0 && i < n;
+    return i;
+}
+
+// Lanes per particle of a launch that does not fill the GPU, so that a push waits
+// for less.  3D: up to a gather group per particle while all blocks are resident,
+// which leaves one round of loads of the group's four; from there, and in 2D, the
+// lanes of a warp only keep one another waiting, which is worth more warps while
+// each scheduler has at most one.  Intervals of 300, 2000, 10 000 and 40 000
+// particles with 1 -> these lanes each: 3D, two frames 2.33 -> 0.77, 2.43 -> 0.83,
+// 2.45 -> 1.16 and 2.82 -> 2.12 ms; 2D 0.78 -> 0.63, 0.80 -> 0.68 and no change.
+// Past these lines: 2D, 40 000 particles, 2 lanes 0.88 -> 1.08 ms; 3D, 2000 particles,
+// 32 lanes 0.83 -> 0.99 ms.
+int spread_of(int ndim, int64_t n, int sm_count) {
+    const int64_t one = (int64_t)sm_count * 128;
+    int sp = 1;
+    while (ndim == 3 && sp < 4 && n * 2 * sp <= one * GPAT_MIXED_MINB_3D) sp *= 2;
+    while (sp < 32 && n * 2 * sp <= one) sp *= 2;
+    return sp;
+}
+
 template <int NDIM, bool NLGC>
 __global__ void __launch_bounds__(128, NDIM == 2 ? GPAT_MIXED_MINB_2D : GPAT_MIXED_MINB_3D)
     mover_mixed_kernel(const MixedRunArgs a, const MixedConsts k, const DevParticles P,
-                       const int64_t n) {
+                       const int64_t n, const int spread) {
     __shared__ __align__(16) float gather[4][kGatherBuf<NDIM>];
-    const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    bool valid;
+    const int64_t i = spread_index(spread, n, valid);
     bool paused;
-    const uint32_t pushes = move_warp<NDIM, NLGC>(a, k, P, i, i < n, paused, a.chunk_pushes,
+    const uint32_t pushes = move_warp<NDIM, NLGC>(a, k, P, i, valid, paused, a.chunk_pushes,
                                                   gather[threadIdx.x >> 5]);
     add_warp_counters(a.cnt, pushes, paused, nullptr);
 }
@@ -76,18 +102,19 @@ __global__ void __launch_bounds__(128, NDIM == 2 ? GPAT_MIXED_MINB_2D : GPAT_MIX
 template <int NDIM, bool NLGC>
 __global__ void __launch_bounds__(128, NDIM == 2 ? GPAT_MIXED_MINB_2D : GPAT_MIXED_MINB_3D)
     mover_learned_kernel(const MixedRunArgs a, const MixedConsts k, const DevParticles P,
-                         const int64_t n, const FusedLearn L) {
+                         const int64_t n, const int spread, const FusedLearn L) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     mma_mlp::SmemInf &S = *reinterpret_cast<mma_mlp::SmemInf *>(smem_raw);
     mma_mlp::load_smem(L.w16, S, false);
     __syncthreads();
     __shared__ __align__(16) float gather[4][kGatherBuf<NDIM>];
-    const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    bool valid;
+    const int64_t i = spread_index(spread, n, valid);
     bool paused;
-    const uint32_t pushes = move_warp<NDIM, NLGC>(a, k, P, i, i < n, paused, a.chunk_pushes,
+    const uint32_t pushes = move_warp<NDIM, NLGC>(a, k, P, i, valid, paused, a.chunk_pushes,
                                                   gather[threadIdx.x >> 5]);
     add_warp_counters(a.cnt, pushes, paused, nullptr);
-    const bool fin = i < n && !paused && P.count_flag[i] == 1;
+    const bool fin = valid && !paused && P.count_flag[i] == 1;
     if (!__any_sync(0xffffffffu, fin)) return;
     float h0[kMlpFeatures];
     if (fin) {
@@ -186,34 +213,35 @@ MixedRunArgs mixed_run_args(const MoverArgs &a) {
 
 cudaError_t launch_mover_mixed(const MoverArgs &a, const MixedConsts &c, int sm_count,
                                cudaStream_t s) {
-    (void)sm_count;
     if (a.n <= 0) return cudaSuccess;
     const int threads = 128;
-    const int64_t blocks = (a.n + threads - 1) / threads;
+    const int sp = spread_of(a.ndim, a.n, sm_count);
+    const int64_t blocks = (a.n * sp + threads - 1) / threads;
     const unsigned g = (unsigned)blocks;
     const MixedRunArgs r = mixed_run_args(a);
     if (a.ndim == 2) {
-        if (a.nlgc) mover_mixed_kernel<2, true><<<g, threads, 0, s>>>(r, c, a.P, a.n);
-        else mover_mixed_kernel<2, false><<<g, threads, 0, s>>>(r, c, a.P, a.n);
+        if (a.nlgc) mover_mixed_kernel<2, true><<<g, threads, 0, s>>>(r, c, a.P, a.n, sp);
+        else mover_mixed_kernel<2, false><<<g, threads, 0, s>>>(r, c, a.P, a.n, sp);
     } else {
-        if (a.nlgc) mover_mixed_kernel<3, true><<<g, threads, 0, s>>>(r, c, a.P, a.n);
-        else mover_mixed_kernel<3, false><<<g, threads, 0, s>>>(r, c, a.P, a.n);
+        if (a.nlgc) mover_mixed_kernel<3, true><<<g, threads, 0, s>>>(r, c, a.P, a.n, sp);
+        else mover_mixed_kernel<3, false><<<g, threads, 0, s>>>(r, c, a.P, a.n, sp);
     }
     return cudaGetLastError();
 }
 
 cudaError_t launch_mover_learned(const MoverArgs &a, const MixedConsts &c, const FusedLearn &L,
-                                 cudaStream_t s) {
+                                 int sm_count, cudaStream_t s) {
     if (a.n <= 0) return cudaSuccess;
-    const unsigned g = (unsigned)((a.n + 127) / 128);
+    const int sp = spread_of(a.ndim, a.n, sm_count);
+    const unsigned g = (unsigned)((a.n * sp + 127) / 128);
     const size_t smem = sizeof(mma_mlp::SmemInf);
     const MixedRunArgs r = mixed_run_args(a);
     if (a.ndim == 2) {
-        if (a.nlgc) mover_learned_kernel<2, true><<<g, 128, smem, s>>>(r, c, a.P, a.n, L);
-        else mover_learned_kernel<2, false><<<g, 128, smem, s>>>(r, c, a.P, a.n, L);
+        if (a.nlgc) mover_learned_kernel<2, true><<<g, 128, smem, s>>>(r, c, a.P, a.n, sp, L);
+        else mover_learned_kernel<2, false><<<g, 128, smem, s>>>(r, c, a.P, a.n, sp, L);
     } else {
-        if (a.nlgc) mover_learned_kernel<3, true><<<g, 128, smem, s>>>(r, c, a.P, a.n, L);
-        else mover_learned_kernel<3, false><<<g, 128, smem, s>>>(r, c, a.P, a.n, L);
+        if (a.nlgc) mover_learned_kernel<3, true><<<g, 128, smem, s>>>(r, c, a.P, a.n, sp, L);
+        else mover_learned_kernel<3, false><<<g, 128, smem, s>>>(r, c, a.P, a.n, sp, L);
     }
     return cudaGetLastError();
 }

@@ -14,11 +14,11 @@ pytestmark = pytest.mark.gpu
 KEYS = ("x", "y", "z", "p", "t", "dt", "count_flag", "nsteps_pushed", "rng_ctr")
 
 
-def _engine(ndim, two):
+def _engine(ndim, two, nmax=200):
     n = 20 if ndim == 3 else 36
     cfg = make_mhd_config(n, n, n if ndim == 3 else 1, 0.0, 1.0, 0.0, 1.0, dt_out=0.02, ndim=ndim)
     prm = make_params(ndim=ndim, p0=0.1, pmin=0.1, pmax=1.0, kpara0=3e-3, kret=0.1, dt_min_rel=1e-2,
-                      dt_max_rel=1e-1, pbcx=1, pbcy=0, pbcz=0, nptl_max=200, seed=5, precision=1,
+                      dt_max_rel=1e-1, pbcx=1, pbcy=0, pbcz=0, nptl_max=nmax, seed=5, precision=1,
                       time_interp=int(two), bin_interval=16)
     eng = Engine(prm, cfg, 0)
     eng.set_tstamps(np.arange(3) * 0.02)
@@ -60,4 +60,29 @@ def test_a_particle_does_not_depend_on_its_neighbours(ndim, two):
         for t, p in got.items():
             for k in KEYS:
                 assert p[k] == alone[t][k] or (p[k] != p[k] and alone[t][k] != alone[t][k]), (t, k)
+    eng.close()
+
+
+@pytest.mark.parametrize("ndim,two", [(2, False), (3, False), (3, True)])
+def test_a_particle_does_not_depend_on_the_lanes_of_a_launch(ndim, two):
+    """Launches that give a particle 1 to 32 lanes, at both sides of each line
+    on 152 SMs: the bits are those of the particle in the whole set."""
+    eng = _engine(ndim, two, 80000)
+    eng.inject_particles_spatial_uniform(80000, 1e-6, 2, 1.0, 1, (0.0, 0.0, 0.0, 1.0, 1.0, 1.0), 1.0)
+    start = eng.get_particles()
+
+    def moved(idx):
+        eng.put_particles(start.take(idx))
+        eng.particle_mover(mhd_tframe=1)
+        out = eng.get_particles()
+        order = np.argsort(out["tag_injected"], kind="stable")
+        return {k: out[k][order] for k in KEYS + ("tag_injected",)}
+
+    whole = moved(np.arange(80000))
+    for n in (38913, 38912, 19457, 19456, 9729, 9728, 4865, 2432, 1217, 1216, 608, 33, 1):
+        idx = np.sort(np.random.default_rng(n).permutation(80000)[:n])
+        got = moved(idx)
+        at = np.isin(whole["tag_injected"], start["tag_injected"][idx])
+        for k in KEYS + ("tag_injected",):
+            assert np.array_equal(got[k], whole[k][at]), (n, k)
     eng.close()
