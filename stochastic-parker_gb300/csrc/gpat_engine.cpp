@@ -1307,6 +1307,17 @@ int gpat_put_particles(gpat_handle_t *h, const gpat_particles_t *src, int64_t n)
     CK(cp(D.tag_injected, src->tag_injected, 4 * c));
     CK(cp(D.tag_splitted, src->tag_splitted, 4 * c));
     CK(cp(D.rng_ctr, src->rng_ctr, 4 * c));
+    // The range of the tags.  On the host it takes 0.7 ns a particle after the
+    // copies, on the GPU a launch and two small copies, about as long as 16 000
+    // particles (put of 1e5 particles 0.22 -> 0.15 ms, of 2e6 2.55 -> 1.03 ms).
+    // Not on the host while the copies run: both then slow down (14.1 ms).
+    const bool on_gpu = n > 16384;
+    if (on_gpu) {
+        CK(cudaMemsetAsync(&h->dcnt->tag_top, 0, 2 * sizeof(unsigned int), h->stream));
+        CK(launch_tag_range(D, n, h->dcnt, h->stream));
+        CK(cudaMemcpyAsync(&h->hcnt.tag_top, &h->dcnt->tag_top, 2 * sizeof(unsigned int),
+                           cudaMemcpyDeviceToHost, h->stream));
+    }
     CK(cudaStreamSynchronize(h->stream));
     h->n = n;
     h->unsorted = true;
@@ -1314,7 +1325,11 @@ int gpat_put_particles(gpat_handle_t *h, const gpat_particles_t *src, int64_t n)
     // injections do not repeat a tag and per-tag tables (labels of learned
     // splitting) cover them
     int64_t top = -1, low = 0;
-    for (int64_t i = 0; i < n; ++i) {
+    if (on_gpu) {
+        top = (int64_t)h->hcnt.tag_top - 1;
+        low = -(int64_t)h->hcnt.tag_low;
+    }
+    for (int64_t i = 0; i < n && !on_gpu; ++i) {
         top = std::max<int64_t>(top, src->tag_injected[i]);
         low = std::min<int64_t>(low, src->tag_splitted[i]);
     }

@@ -54,6 +54,7 @@ struct DevCounters {
     // per frame slot: some field value (or fluctuation value) is subnormal,
     // infinite or NaN
     unsigned int odd_fields[2], odd_aux[2];
+    unsigned int tag_top, tag_low;   // launch_tag_range
 };
 
 // Packed per-cell field records read by the movers (see fields.cu for the slot
@@ -251,6 +252,9 @@ cudaError_t launch_calc_aux_gradients(float *aux, int ndim, int nxg, int nyg, in
 cudaError_t launch_scatter_aux(const float *src, float *aux, int comp, size_t ncells,
                                cudaStream_t s);
 cudaError_t launch_fill(float *a, float v, size_t n, cudaStream_t s);
+// Raises cnt->tag_top to the largest tag_injected + 1 and cnt->tag_low to the
+// largest -tag_splitted, where these are above 0.
+cudaError_t launch_tag_range(const DevParticles &P, int64_t n, DevCounters *cnt, cudaStream_t s);
 cudaError_t launch_mover_fp64(const MoverArgs &a, int sm_count, cudaStream_t s);
 // The same in teams of kMoverTeam lanes, for launch_mover_fp64.
 constexpr int kMoverTeam = 8;

@@ -1343,6 +1343,33 @@ cudaError_t launch_quick_check(const DevParticles &P, int64_t n, DevCounters *cn
 
 namespace {
 
+__global__ void __launch_bounds__(256) tag_range_kernel(const DevParticles P, int64_t n,
+                                                        DevCounters *cnt) {
+    unsigned top = 0, low = 0;
+    for (int64_t i = (int64_t)blockIdx.x * 256 + threadIdx.x; i < n; i += 256ll * gridDim.x) {
+        const int t = P.tag_injected[i], l = P.tag_splitted[i];
+        if (t >= 0) top = max(top, (unsigned)t + 1u);
+        if (l < 0) low = max(low, 0u - (unsigned)l);
+    }
+    top = __reduce_max_sync(0xffffffffu, top);
+    low = __reduce_max_sync(0xffffffffu, low);
+    if ((threadIdx.x & 31) == 0) {
+        if (top) atomicMax(&cnt->tag_top, top);
+        if (low) atomicMax(&cnt->tag_low, low);
+    }
+}
+
+}  // namespace
+
+cudaError_t launch_tag_range(const DevParticles &P, int64_t n, DevCounters *cnt, cudaStream_t s) {
+    if (n <= 0) return cudaSuccess;
+    const unsigned g = (unsigned)std::min<int64_t>((n + 255) / 256, 608);
+    tag_range_kernel<<<g, 256, 0, s>>>(P, n, cnt);
+    return cudaGetLastError();
+}
+
+namespace {
+
 // get_ncells_large_* (mhd_data_parallel.f90:2211-2498) over the nodes
 // ix = 1..nx (position xmin + (ix - 1) dx), single-precision quantities as
 // the reference's real(sp) arrays give them.
