@@ -252,21 +252,20 @@ def measured_peaks() -> dict:
 # density, and the L1TEX throughput (percent of peak, active cycles) of the
 # full capture, which ncu names as the binding unit of the gather movers.
 NCU_MOVER = {
-    ("global", 2): {"dram_bytes_per_push": 0.934, "l1tex_pct": 94.2,
-                    "profile": "profiles/mover_mixed_turbulent_shock_2d.md"},
-    ("global", 3): {"dram_bytes_per_push": 6.7, "l1tex_pct": 91.7,
-                    "profile": "profiles/mover_mixed_turbulence_3d.md"},
+    ("global", 2): {"dram_bytes_per_push": 0.934, "l1tex_pct": 71.5,
+                    "profile": "profiles/case_times.md"},
+    ("global", 3): {"dram_bytes_per_push": 6.7, "l1tex_pct": 71.6,
+                    "profile": "profiles/case_times.md"},
 }
-# The L1TEX data path per push and per clock.  Global-gather movers: the
-# 32-byte loads of scattered records cost one data-pipe wavefront per
-# 32-byte sector (3D capture: 1.51e9 wavefronts for 1.53e9 sectors; the pipe
-# at 88 % of its wavefronts), one wavefront per clock per SM, so the rate is
-# sectors: 7.3 per push in 2D (8 loads, neighbouring lanes share some), 24
-# in 3D (8 corners x 3 loads; 23.0 distinct sectors per 32-lane request).
-# Brick movers read 16-byte chunks from shared memory, up to 128 bytes per
-# wavefront (nominal; bank conflicts cost more).
-L1_MODEL = {("global", 2): {"bytes_per_push": 7.3 * 32, "bytes_per_clk_sm": 32},
-            ("global", 3): {"bytes_per_push": 24 * 32, "bytes_per_clk_sm": 32},
+# The L1TEX data path per push and per clock, in data-pipe wavefronts of up to
+# 128 bytes, one per clock per SM.  Global-gather movers: groups of lanes read
+# a record's sectors of one line together, and the captures count 4.35
+# wavefronts per push in 2D (1.114e9 for 2.56e8 pushes) and about 14 in 3D
+# (1.189e9 for 8.5e7, the exchange through shared memory included).  Brick
+# movers read 16-byte chunks from shared memory (nominal; bank conflicts cost
+# more).
+L1_MODEL = {("global", 2): {"bytes_per_push": 4.35 * 128, "bytes_per_clk_sm": 128},
+            ("global", 3): {"bytes_per_push": 14 * 128, "bytes_per_clk_sm": 128},
             ("tile", 2): {"bytes_per_push": 4 * 64, "bytes_per_clk_sm": 128},
             ("tile", 3): {"bytes_per_push": 8 * (5 * 16 + 4), "bytes_per_clk_sm": 128}}
 
@@ -281,13 +280,9 @@ def roofline_of(kind, ndim, avg_ms, avg_steps, avg_n, sm_count, sm_mhz, peaks) -
     alg = avg_steps * GATHER_BYTES_PER_STEP[ndim] + avg_n * STATE_BYTES_PER_PARTICLE
     ncu = NCU_MOVER.get((kind, ndim), {})
     dram = ncu.get("dram_bytes_per_push")
-    if m["bytes_per_clk_sm"] == 32:
-        peak_source = (f"L1TEX data pipe: one 32-byte sector per clock per SM for scattered "
-                       f"32-byte loads (ncu: wavefronts = sectors) x {sm_count} SMs x median "
-                       f"sampled SM clock {sm_mhz} MHz")
-    else:
-        peak_source = (f"nominal shared-memory rate: 128 B/clk per SM x {sm_count} SMs x "
-                       f"median sampled SM clock {sm_mhz} MHz")
+    what = "L1TEX data pipe" if kind == "global" else "nominal shared-memory rate"
+    peak_source = (f"{what}: one wavefront of 128 bytes per clock per SM x {sm_count} SMs x "
+                   f"median sampled SM clock {sm_mhz} MHz")
     return {"bound": "l1", "achieved": l1_bytes / secs / 1e9, "peak": l1_peak, "unit": "GB/s",
             "frac": l1_bytes / secs / 1e9 / l1_peak, "peak_source": peak_source,
             "traffic": dram * avg_steps if dram is not None else None,
@@ -300,8 +295,8 @@ def roofline_of(kind, ndim, avg_ms, avg_steps, avg_n, sm_count, sm_mhz, peaks) -
                     "frac": alg / secs / 1e9 / peaks["hbm_gbs"], "peak_source": peaks["source"],
                     "algorithmic_bytes_per_push": GATHER_BYTES_PER_STEP[ndim],
                     "state_bytes_per_particle": STATE_BYTES_PER_PARTICLE},
-            "note": "achieved = L1 sectors (32 B) the gathers move per push x pushes / launch "
-                    "time, against the data pipe's sector rate; ncu_l1tex_throughput_pct is the "
+            "note": "achieved = L1 data-pipe wavefronts (128 B) per push x pushes / launch "
+                    "time, against one per clock and SM; ncu_l1tex_throughput_pct is the "
                     "unit's measured busy share; hbm = algorithmic bytes (corners x stored field "
                     "arrays x 4 B + FP64 state) over measured HBM"}
 
