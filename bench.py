@@ -249,12 +249,12 @@ def measured_peaks() -> dict:
 
 # From the ncu captures summarised in profiles/ (commands there): DRAM bytes
 # (read + write) per push of the mover kernel at the bench's particle
-# density, and the L1TEX throughput (percent of peak, active cycles) of the
+# density (3D: two late launches of 3e7 particles), and the L1TEX throughput (percent of peak, active cycles) of the
 # full capture, which ncu names as the binding unit of the gather movers.
 NCU_MOVER = {
-    ("global", 2): {"dram_bytes_per_push": 0.934, "l1tex_pct": 71.5,
+    ("global", 2): {"dram_bytes_per_push": 0.947, "l1tex_pct": 71.5,
                     "profile": "profiles/case_times.md"},
-    ("global", 3): {"dram_bytes_per_push": 6.7, "l1tex_pct": 71.6,
+    ("global", 3): {"dram_bytes_per_push": 44.0, "l1tex_pct": 71.6,
                     "profile": "profiles/case_times.md"},
 }
 # The L1TEX data path per push and per clock, in data-pipe wavefronts of up to

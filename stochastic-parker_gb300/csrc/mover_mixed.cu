@@ -18,7 +18,8 @@
 // reference's (2u-1)*sqrt(3) variates (or Gaussian), four from one
 // Philox-4x32-10 call per push.  The per-particle body is in mixed_body.cuh;
 // this file holds the kernels that gather the packed field records from
-// global memory (one particle per thread, and the batched persistent form).
+// global memory (one particle per thread where a launch fills the GPU, and the
+// batched persistent form).
 #include "mixed_body.cuh"
 
 #include "learned_dev.cuh"
