@@ -8,9 +8,8 @@ namespace gpat {
 // Slot order of the packed records, as indices into the 32-variable cell
 // (vars 0-7: vx vy vz rho bx by bz |B|; gradient of var v along d at 8+3v+d).
 __constant__ int kPack2D[kRec2D] = {0, 1, 4, 5, 6, 8, 12, 20, 21, 23, 24, 26, 27, 29, 30, 3};
-__constant__ int kPack3D[kRec3D] = {0,  1,  2,  4,  5,  6,  8,  12, 16, 20, 21,
-                                    22, 23, 24, 25, 26, 27, 28, 29, 30, 31, 3,
-                                    7,  -1, -1, -1, -1, -1, -1, -1, -1, -1};
+__constant__ int kPack3D[kRec3D] = {0, 1, 2, 4, 5, 6, 8, 12, 16, 20, 21, 22,
+                                    23, 24, 25, 26, 27, 28, 29, 30, 31, 3, 7, -1};
 
 // One 16-byte chunk of the 32-variable record per thread: HBM streaming (32 B
 // read, 128 B written per cell) with full lines written.
@@ -136,7 +135,7 @@ struct GradArgs {
 // Gradients (GRAD) and packed records, eight lanes per cell: lane v takes the
 // derivatives of variable v, the cell's 32 values meet in shared memory, and
 // each lane then writes one 16-byte chunk of the gradients and of the record.
-// HBM streaming: 32 B read and 96 + 64 (2D) or 128 (3D) B written per cell.
+// HBM streaming: 32 B read and 96 + 64 (2D) or 96 (3D) B written per cell.
 // One thread per cell with scalar stores at a stride of 128 bytes took 1055 us
 // for the gradients of 132^3 cells, 564 us for the records.
 template <int R, bool GRAD>
@@ -300,17 +299,16 @@ namespace gpat {
 namespace {
 
 // Chunk-planar copy of the packed records: float4 chunk j of every node
-// contiguous, planes[j * ncells + c] = rec[c * R + 4 j .. 4 j + 3], without
-// the 3D records' padding.  The
+// contiguous, planes[j * ncells + c] = rec[c * R + 4 j .. 4 j + 3].  The
 // tile mover stages these planes, so neighbouring nodes of one chunk sit in
 // neighbouring shared-memory bank groups.
-template <int R, int CHUNKS>
+template <int R>
 __global__ void planarize_kernel(const float4 *__restrict__ rec, float4 *__restrict__ planes,
                                  size_t ncells) {
     const size_t stride = (size_t)gridDim.x * blockDim.x;
     for (size_t c = (size_t)blockIdx.x * blockDim.x + threadIdx.x; c < ncells; c += stride) {
 #pragma unroll
-        for (int j = 0; j < CHUNKS; ++j) planes[(size_t)j * ncells + c] = rec[c * (R / 4) + j];
+        for (int j = 0; j < R / 4; ++j) planes[(size_t)j * ncells + c] = rec[c * (R / 4) + j];
     }
 }
 
@@ -323,8 +321,8 @@ cudaError_t launch_planarize_records(const float *rec, float *planes, int ndim, 
     if (blocks > 65535 * 8) blocks = 65535 * 8;
     const float4 *r = reinterpret_cast<const float4 *>(rec);
     float4 *o = reinterpret_cast<float4 *>(planes);
-    if (ndim == 2) planarize_kernel<kRec2D, kChunks2D><<<(unsigned)blocks, threads, 0, s>>>(r, o, ncells);
-    else planarize_kernel<kRec3D, kChunks3D><<<(unsigned)blocks, threads, 0, s>>>(r, o, ncells);
+    if (ndim == 2) planarize_kernel<kRec2D><<<(unsigned)blocks, threads, 0, s>>>(r, o, ncells);
+    else planarize_kernel<kRec3D><<<(unsigned)blocks, threads, 0, s>>>(r, o, ncells);
     return cudaGetLastError();
 }
 

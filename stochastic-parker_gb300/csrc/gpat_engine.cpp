@@ -1524,7 +1524,7 @@ int gpat_particle_mover(gpat_handle_t *h, int focused_transport, int nlgc, doubl
         s.item_counter = reinterpret_cast<unsigned long long *>(h->tile_dev + s.nbricks + 1);
         s.nodes = (uint32_t)((sx + 1) * (sy + 1) * (h->prm.ndim == 3 ? sz + 1 : 1));
         // chunk-planar copies of the frames' records, rebuilt when the records changed
-        const int R = 4 * ((h->prm.ndim == 2) ? kChunks2D : kChunks3D);
+        const int R = (h->prm.ndim == 2) ? kRec2D : kRec3D;
         for (int slot = 0; slot < (a.time_interp ? 2 : 1); ++slot) {
             if (!h->planes[slot]) {
                 if (cudaMalloc(&h->planes[slot], (size_t)R * sizeof(float) * h->ncells) !=

@@ -58,14 +58,13 @@ struct DevCounters {
 };
 
 // Packed per-cell field records read by the movers (see fields.cu for the slot
-// order).  2D: 16 floats; 3D: 24 floats, the first 21 of them read, in a
-// 128-byte line of their own: a group of lanes then reads a record's sectors
-// with one tag lookup (2.0e11 random records/s against 1.4e11 at a stride of
-// 96 bytes, where half of the records span two lines).  The brick mover's
-// chunk planes hold the 24 floats.
+// order).  2D: 16 floats; 3D: 24 floats, the first 21 of them read.  3D records
+// in 128-byte lines of their own would take a third more memory (of a frame's 224
+// bytes a cell, 256) for next to nothing: gathered by groups of lanes, at most
+// 1.03 times the rate (1e6 particles on 128^3 cells; 1.00 on 64^3), gathered by
+// single lanes 0.65 to 0.9 of it.
 constexpr int kRec2D = 16;
-constexpr int kRec3D = 32;
-constexpr int kChunks2D = 4, kChunks3D = 6;   // 16-byte chunks with data
+constexpr int kRec3D = 24;
 
 // Particle tracking (track_particle_flag, particle_module.f90:144-150):
 // tags_tracking(nrows, n) and particles_tracked(nsteps_max, n), both in

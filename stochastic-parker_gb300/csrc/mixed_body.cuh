@@ -85,8 +85,8 @@ __device__ __forceinline__ void negp_or_boundary(const MixedRunArgs &a, const Mi
 }
 
 // 256-bit read-only global load (8 floats, 32-byte aligned address).  Records
-// are 64 B (2D) or 96 B in a 128-byte line (3D), so one corner costs 2 or 3 of
-// these instead of 4 or 6 128-bit loads.
+// are 64 B (2D) or 96 B (3D) at 32-byte aligned offsets, so one corner costs 2
+// or 3 of these instead of 4 or 6 128-bit loads.
 __device__ __forceinline__ void ld8(const float *p, float (&v)[8]) {
     asm("ld.global.nc.v8.f32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
         : "=f"(v[0]), "=f"(v[1]), "=f"(v[2]), "=f"(v[3]), "=f"(v[4]), "=f"(v[5]), "=f"(v[6]),
@@ -162,8 +162,9 @@ __device__ __forceinline__ bool interp_global(const MixedRunArgs &a, const Pos &
 // corner's record for every particle of the group in turn, weighs and sums it,
 // and the sums change hands.  A load instruction then touches
 // 16 (8) lines instead of 32 scattered sectors, and the L1 data pipe, which
-// spends a wavefront per line touched, delivers twice the records (random
-// records of 64 B: 2.3e11/s against 1.15e11; of 96 B: 1.96e11 against 9.9e10).
+// spends a wavefront per line touched, delivers more records (random records of
+// 64 B: 2.3e11/s against 1.15e11; of 96 B, half of which span two lines: 1.4e11
+// against 9.9e10).
 // Weights and the order of the sums are interp_global's.  want: the lane's
 // particle makes a push.  All lanes of the warp call; buf: its kGatherBuf<NDIM>
 // floats.  False where the position is outside the ghost range.
@@ -352,7 +353,7 @@ struct TileGather {
     template <int NDIM, int NV>
     __device__ __forceinline__ bool interp(const MixedRunArgs &a, const Pos &q, float rt,
                                            float f[NV]) const {
-        constexpr int R4 = (NDIM == 2) ? kChunks2D : kChunks3D;
+        constexpr int R4 = ((NDIM == 2) ? kRec2D : kRec3D) / 4;
         const int ix = q.cx + 2, iy = q.cy + 2, iz = (NDIM == 3) ? q.cz + 2 : 0;
         if ((unsigned)ix > (unsigned)(a.nxg - 2) || (unsigned)iy > (unsigned)(a.nyg - 2) ||
             (NDIM == 3 && (unsigned)iz > (unsigned)(a.nzg - 2))) {

@@ -280,7 +280,7 @@ cudaError_t launch_tile(const MixedRunArgs &r, const MixedConsts &c, const DevPa
 
 size_t tile_smem_bytes(int ndim, int sx, int sy, int sz, int time_interp, uint32_t *tile_bytes,
                        uint32_t *tile2_off) {
-    const size_t rec = (size_t)((ndim == 2) ? kChunks2D : kChunks3D) * sizeof(float4);
+    const size_t rec = (size_t)((ndim == 2) ? kRec2D : kRec3D) * sizeof(float);
     const size_t nodes = (size_t)(sx + 1) * (sy + 1) * (ndim == 3 ? sz + 1 : 1);
     const size_t one = nodes * rec;
     const size_t off = (one + 127) & ~(size_t)127;   // frame 2 at a 128-byte boundary
@@ -302,7 +302,7 @@ cudaError_t encode_brick_map(CUtensorMap *m, const float *planes, int ndim, int 
         encode = reinterpret_cast<PFN_cuTensorMapEncodeTiled_v12000>(fn);
     }
     // planes: [R/4][nzg][nyg][nxg] float4; dims innermost first
-    const cuuint64_t nch = (ndim == 2) ? kChunks2D : kChunks3D;
+    const cuuint64_t nch = ((ndim == 2) ? kRec2D : kRec3D) / 4;
     const cuuint64_t nx = (cuuint64_t)nxg, ny = (cuuint64_t)nyg, nz = (cuuint64_t)nzg;
     cuuint64_t dims[5], strides[4];
     cuuint32_t box[5];
