@@ -635,7 +635,13 @@ __device__ __forceinline__ uint32_t move_particle(const MixedRunArgs &a, const M
         while (alive && target_d < a.limit) {
             const float target = (float)target_d;
             while (tau - tc < target && flag == 1) {
+                // Lanes whose particle is outside the box's cells would stay apart
+                // for the push: they meet the others again.  Brick mover, steps of
+                // half a cell, 3D 64^3: 41.4 -> 35.7 ms (37.6 with every lane through
+                // the boundary test); 2D 64^2: 58.6 -> 54.9 (56.6).
+                const unsigned here = __activemask();
                 negp_or_boundary<NDIM>(a, k, q, p - pc, flag, wp);
+                __syncwarp(here);
                 if (flag != 1) break;
                 if (limit != 0 && pushes >= limit) {
                     paused = true;   // between pushes: the next launch resumes from t
