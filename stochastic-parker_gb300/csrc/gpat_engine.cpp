@@ -2113,7 +2113,8 @@ struct gpat_batch {
     unsigned long long *host_ull = nullptr;   // pinned: run_n readback and nactive
     std::vector<BatchRun> desc;
     cudaGraphExec_t exec[2] = {nullptr, nullptr};
-    int graph_key[3] = {-1, -1, -1};       // nlgc, minb, grab of the captured graphs
+    bool group = true;                     // gather form of the next call
+    int graph_key[4] = {-1, -1, -1, -1};   // nlgc, minb, grab, group of the captured graphs
     std::vector<void *> graph_scratch;     // each run's binning scratch in the graphs
     gpat_batch_tuning_t tuning{};
     std::string err;
@@ -2145,7 +2146,7 @@ void destroy_graphs(gpat_batch_t *b) {
         if (e) cudaGraphExecDestroy(e);
         e = nullptr;
     }
-    b->graph_key[0] = b->graph_key[1] = b->graph_key[2] = -1;
+    std::fill(std::begin(b->graph_key), std::end(b->graph_key), -1);
 }
 
 // Captures the chunk graph for both buffer parities: scheduler prefix, the
@@ -2159,7 +2160,7 @@ int capture_graphs(gpat_batch_t *b, int nlgc, int minb, int grab) {
         cudaError_t e = launch_batch_prefix(nr, run_n_dev(b), b->tile_prefix, tile_counter_dev(b),
                                             nactive_dev(b), b->stream);
         if (e == cudaSuccess)
-            e = launch_mover_mixed_batch(b->ndim, nlgc != 0, minb, parity, nr, b->sm_count, grab,
+            e = launch_mover_mixed_batch(b->ndim, nlgc != 0, minb, b->group, parity, nr, b->sm_count, grab,
                                          b->tile_prefix, run_n_dev(b), tile_counter_dev(b),
                                          nactive_dev(b), b->stream);
         for (int r = 0; r < nr && e == cudaSuccess; ++r) {
@@ -2184,6 +2185,7 @@ int capture_graphs(gpat_batch_t *b, int nlgc, int minb, int grab) {
     b->graph_key[0] = nlgc;
     b->graph_key[1] = minb;
     b->graph_key[2] = grab;
+    b->graph_key[3] = b->group ? 1 : 0;
     b->graph_scratch.clear();
     for (gpat_handle_t *h : b->runs) b->graph_scratch.push_back(h->sort_scratch);
     return GPAT_OK;
@@ -2195,9 +2197,11 @@ int batch_prepare(gpat_batch_t *b, const int *tframes, int nlgc, double kperp_kp
                   int nsteps_interval, int num_fine_steps) {
     const int nr = (int)b->runs.size();
     b->desc.resize(nr);
+    std::vector<MoverArgs> args(nr);
+    int64_t grouped = 0, total = 0;   // particles by the form their run gains from
     for (int r = 0; r < nr; ++r) {
         gpat_handle_t *h = b->runs[r];
-        MoverArgs a;
+        MoverArgs &a = args[r];
         int rc = mover_args(h, tframes[r], nsteps_interval, num_fine_steps, a);
         if (rc) return bfail(b, rc, "run " + std::to_string(r) + ": " + h->err);
         a.nlgc = nlgc ? 1 : 0;
@@ -2218,7 +2222,11 @@ int batch_prepare(gpat_batch_t *b, const int *tframes, int nlgc, double kperp_kp
         d.P[0] = h->P[0];
         d.P[1] = h->P[1];
         b->host_ull[r] = (unsigned long long)h->n;
+        total += h->n;
     }
+    for (int r = 0; r < nr; ++r)
+        if (mover_gathers_in_groups(args[r], total, b->sm_count)) grouped += b->runs[r]->n;
+    b->group = 2 * grouped >= total;
     BCK(upload_batch_runs(b->desc.data(), nr, b->stream));
     BCK(cudaMemcpyAsync(run_n_dev(b), b->host_ull, sizeof(unsigned long long) * (size_t)nr,
                         cudaMemcpyHostToDevice, b->stream));
@@ -2338,7 +2346,7 @@ int gpat_batch_particle_mover(gpat_batch_t *b, const int *mhd_tframe, int nlgc, 
     for (size_t r = 0; same_scratch && r < b->runs.size(); ++r)
         same_scratch = b->graph_scratch[r] == b->runs[r]->sort_scratch;
     if (!b->exec[0] || b->graph_key[0] != (nlgc ? 1 : 0) || b->graph_key[1] != b->tuning.minb ||
-        b->graph_key[2] != b->tuning.grab || !same_scratch) {
+        b->graph_key[2] != b->tuning.grab || b->graph_key[3] != (b->group ? 1 : 0) || !same_scratch) {
         rc = capture_graphs(b, nlgc ? 1 : 0, b->tuning.minb, b->tuning.grab);
         if (rc) return rc;
     }

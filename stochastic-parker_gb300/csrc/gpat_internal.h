@@ -268,6 +268,9 @@ MixedConsts make_mixed_consts(const MoverArgs &a);
 // The global-gather chunk launch with learned splitting of finished particles.
 cudaError_t launch_mover_learned(const MoverArgs &a, const MixedConsts &c, const FusedLearn &L,
                                  int sm_count, cudaStream_t s);
+// Whether a launch of n particles, a.n of them of this run, gathers by groups of
+// lanes (gather_form.h).
+bool mover_gathers_in_groups(const MoverArgs &a, int64_t n, int sm_count);
 MixedRunArgs mixed_run_args(const MoverArgs &a);
 // Batched split-precision mover (see mover_mixed.cu).
 cudaError_t upload_batch_runs(const BatchRun *runs, int nruns, cudaStream_t s);
@@ -283,7 +286,7 @@ cudaError_t launch_cell_sort_dev(const DevParticles &src, const DevParticles &ds
                                  unsigned long long *n_dev, int64_t cap, const CellGrid &g,
                                  void *scratch, DevCounters *cnt, const EscHist &esc,
                                  cudaStream_t s);
-cudaError_t launch_mover_mixed_batch(int ndim, bool nlgc, int minb, int parity, int nruns,
+cudaError_t launch_mover_mixed_batch(int ndim, bool nlgc, int minb, bool group, int parity, int nruns,
                                      int sm_count, int grab, const long long *tile_prefix,
                                      const unsigned long long *run_n,
                                      unsigned long long *tile_counter,

@@ -757,14 +757,14 @@ __device__ __forceinline__ int next_nsp(int nsp, int interval) {
     return n == interval ? 0 : n % interval;
 }
 
-// move_particle with the gathers of a whole warp (interp_group): the loop turns
-// once per push of the warp, ordinary and landing pushes through the same
-// code, until no lane's particle has one left before its pause or the end of
-// the interval.  All lanes call; i, valid: the lane's particle; paused: it has
-// pushes left.  (Lanes that take another particle when theirs is done, as the
+// move_particle for a whole warp: the loop turns once per push of the warp,
+// ordinary and landing pushes through the same code, until no lane's particle has
+// one left before its pause or the end of the interval.  GROUP: gathers by groups
+// of lanes (interp_group), else each lane its own.  All lanes call; i, valid: the
+// lane's particle; paused: it has pushes left.  (Lanes that take another particle when theirs is done, as the
 // FP64 mover's do, lose more in shared records than they gain: 3D 29.8 against
 // 24.3 ms for 1e6 particles, 2D 43.8 against 39.3 for 2e6.)
-template <int NDIM, bool NLGC>
+template <int NDIM, bool NLGC, bool GROUP>
 __device__ __forceinline__ uint32_t move_warp(const MixedRunArgs &a, const MixedConsts &k,
                                               const DevParticles &P, int64_t i, bool valid,
                                               bool &paused, uint32_t limit, float *buf) {
@@ -858,7 +858,9 @@ __device__ __forceinline__ uint32_t move_warp(const MixedRunArgs &a, const Mixed
         }
         if (!__any_sync(0xffffffffu, want)) break;
         float f[NV];
-        const bool ok = interp_group<NDIM, NV>(a, q, tau * k.inv_dtf, want, buf, f);
+        bool ok = false;
+        if (GROUP) ok = interp_group<NDIM, NV>(a, q, tau * k.inv_dtf, want, buf, f);
+        else if (want) ok = interp_global<NDIM, NV>(a, q, tau * k.inv_dtf, f);
         if (!want) continue;
         if (!ok) {
             flag = 0;
@@ -929,6 +931,28 @@ __device__ __forceinline__ uint32_t move_warp(const MixedRunArgs &a, const Mixed
     P.nsteps_tracked[i] = 1;
     P.rng_ctr[i] = ctr;
     if (a.pause) a.pause[i] = paused ? 1 : 0;
+    return pushes;
+}
+
+// The particle of each lane of a warp over a chunk, in the form the launch chose
+// (gathers_in_groups).  By single lanes, 2D runs through move_particle, whose two
+// copies of the push need fewer registers than move_warp's loop (256^2 cells, 8 and
+// 2 a cell: 22.9 against 24.3 and 9.0 against 10.0 ms); 3D through the loop, which
+// needs no second copy (128^3, 0.5 a cell, one frame: 11.5 against 12.6 ms).
+template <int NDIM, bool NLGC, bool GROUP>
+__device__ __forceinline__ uint32_t move_lanes(const MixedRunArgs &a, const MixedConsts &k,
+                                               const DevParticles &P, int64_t i, bool valid,
+                                               bool &paused, float *buf) {
+    if (GROUP || NDIM == 3)
+        return move_warp<NDIM, NLGC, GROUP>(a, k, P, i, valid, paused, a.chunk_pushes, buf);
+    uint32_t pushes = 0;
+    bool exited = false;
+    paused = false;
+    if (valid) {
+        pushes = move_particle<NDIM, NLGC>(a, k, P, i, paused, GlobalGather{}, a.chunk_pushes, exited);
+        if (a.pause) a.pause[i] = paused ? 1 : 0;
+    }
+    __syncwarp();
     return pushes;
 }
 

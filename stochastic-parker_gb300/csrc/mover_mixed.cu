@@ -20,6 +20,7 @@
 // this file holds the kernels that gather the packed field records from
 // global memory (one particle per thread where a launch fills the GPU, and the
 // batched persistent form).
+#include "gather_form.h"
 #include "mixed_body.cuh"
 
 #include "learned_dev.cuh"
@@ -81,16 +82,16 @@ int spread_of(int ndim, int64_t n, int sm_count) {
     return sp;
 }
 
-template <int NDIM, bool NLGC>
+template <int NDIM, bool NLGC, bool GROUP>
 __global__ void __launch_bounds__(128, NDIM == 2 ? GPAT_MIXED_MINB_2D : GPAT_MIXED_MINB_3D)
     mover_mixed_kernel(const MixedRunArgs a, const MixedConsts k, const DevParticles P,
                        const int64_t n, const int spread) {
-    __shared__ __align__(16) float gather[4][kGatherBuf<NDIM>];
+    __shared__ __align__(16) float gather[4][GROUP ? kGatherBuf<NDIM> : 1];
     bool valid;
     const int64_t i = spread_index(spread, n, valid);
     bool paused;
-    const uint32_t pushes = move_warp<NDIM, NLGC>(a, k, P, i, valid, paused, a.chunk_pushes,
-                                                  gather[threadIdx.x >> 5]);
+    const uint32_t pushes =
+        move_lanes<NDIM, NLGC, GROUP>(a, k, P, i, valid, paused, gather[threadIdx.x >> 5]);
     add_warp_counters(a.cnt, pushes, paused, nullptr);
 }
 
@@ -100,7 +101,7 @@ __global__ void __launch_bounds__(128, NDIM == 2 ? GPAT_MIXED_MINB_2D : GPAT_MIX
 // to the normalisation of the next interval and applies the weight window
 // (split into lineage-tagged copies appended after the set, or roulette) in
 // the same launch.  Warps with no finished particle skip the network.
-template <int NDIM, bool NLGC>
+template <int NDIM, bool NLGC, bool GROUP>
 __global__ void __launch_bounds__(128, NDIM == 2 ? GPAT_MIXED_MINB_2D : GPAT_MIXED_MINB_3D)
     mover_learned_kernel(const MixedRunArgs a, const MixedConsts k, const DevParticles P,
                          const int64_t n, const int spread, const FusedLearn L) {
@@ -108,12 +109,12 @@ __global__ void __launch_bounds__(128, NDIM == 2 ? GPAT_MIXED_MINB_2D : GPAT_MIX
     mma_mlp::SmemInf &S = *reinterpret_cast<mma_mlp::SmemInf *>(smem_raw);
     mma_mlp::load_smem(L.w16, S, false);
     __syncthreads();
-    __shared__ __align__(16) float gather[4][kGatherBuf<NDIM>];
+    __shared__ __align__(16) float gather[4][GROUP ? kGatherBuf<NDIM> : 1];
     bool valid;
     const int64_t i = spread_index(spread, n, valid);
     bool paused;
-    const uint32_t pushes = move_warp<NDIM, NLGC>(a, k, P, i, valid, paused, a.chunk_pushes,
-                                                  gather[threadIdx.x >> 5]);
+    const uint32_t pushes =
+        move_lanes<NDIM, NLGC, GROUP>(a, k, P, i, valid, paused, gather[threadIdx.x >> 5]);
     add_warp_counters(a.cnt, pushes, paused, nullptr);
     const bool fin = valid && !paused && P.count_flag[i] == 1;
     if (!__any_sync(0xffffffffu, fin)) return;
@@ -145,13 +146,13 @@ __global__ void __launch_bounds__(128, NDIM == 2 ? GPAT_MIXED_MINB_2D : GPAT_MIX
 // ---------------------------------------------------------------------------
 __constant__ BatchRun c_batch_runs[kMaxBatchRuns];
 
-template <int NDIM, bool NLGC, int MINB>
+template <int NDIM, bool NLGC, int MINB, bool GROUP>
 __global__ void __launch_bounds__(128, MINB)
     mover_mixed_batch_kernel(const int parity, const int nruns, const long long *tile_prefix,
                              const unsigned long long *run_n, unsigned long long *tile_counter,
                              const int grab, unsigned long long *nactive_total) {
     __shared__ long long s_tile;
-    __shared__ __align__(16) float gather[4][kGatherBuf<NDIM>];
+    __shared__ __align__(16) float gather[4][GROUP ? kGatherBuf<NDIM> : 1];
     const long long total = tile_prefix[nruns];
     for (;;) {
         __syncthreads();
@@ -171,8 +172,8 @@ __global__ void __launch_bounds__(128, MINB)
             const int64_t i = (t - tile_prefix[lo]) * 128 + threadIdx.x;
             bool paused;
             const uint32_t pushes =
-                move_warp<NDIM, NLGC>(d.a, d.k, d.P[parity], i, i < (int64_t)run_n[lo], paused,
-                                      d.a.chunk_pushes, gather[threadIdx.x >> 5]);
+                move_lanes<NDIM, NLGC, GROUP>(d.a, d.k, d.P[parity], i, i < (int64_t)run_n[lo],
+                                              paused, gather[threadIdx.x >> 5]);
             add_warp_counters(d.a.cnt, pushes, paused, nactive_total);
         }
     }
@@ -212,39 +213,57 @@ MixedRunArgs mixed_run_args(const MoverArgs &a) {
     return r;
 }
 
+bool mover_gathers_in_groups(const MoverArgs &a, int64_t n, int sm_count) {
+    const double cells = (double)a.nxg * a.nyg * a.nzg;
+    return gathers_in_groups({a.ndim, a.time_interp != 0, n, cells, (double)a.n / cells,
+                              gather_step(a.ndim, a.kpara0, a.dt_max, a.dx, a.dy, a.dz), sm_count});
+}
+
+namespace {
+
+template <int NDIM, bool NLGC, bool GROUP>
+void launch_form(const MoverArgs &a, const MixedConsts &c, const FusedLearn *L, int sm_count,
+                 cudaStream_t s) {
+    const int sp = spread_of(NDIM, a.n, sm_count);
+    const unsigned g = (unsigned)((a.n * sp + 127) / 128);
+    const MixedRunArgs r = mixed_run_args(a);
+    if (L)
+        mover_learned_kernel<NDIM, NLGC, GROUP><<<g, 128, sizeof(mma_mlp::SmemInf), s>>>(
+            r, c, a.P, a.n, sp, *L);
+    else
+        mover_mixed_kernel<NDIM, NLGC, GROUP><<<g, 128, 0, s>>>(r, c, a.P, a.n, sp);
+}
+
+cudaError_t launch_mover(const MoverArgs &a, const MixedConsts &c, const FusedLearn *L,
+                         int sm_count, cudaStream_t s) {
+    if (a.n <= 0) return cudaSuccess;
+    const bool group = mover_gathers_in_groups(a, a.n, sm_count);
+#define GPAT_FORM(ND, NL)                                          \
+    do {                                                           \
+        if (group) launch_form<ND, NL, true>(a, c, L, sm_count, s); \
+        else launch_form<ND, NL, false>(a, c, L, sm_count, s);      \
+    } while (0)
+    if (a.ndim == 2) {
+        if (a.nlgc) GPAT_FORM(2, true);
+        else GPAT_FORM(2, false);
+    } else {
+        if (a.nlgc) GPAT_FORM(3, true);
+        else GPAT_FORM(3, false);
+    }
+#undef GPAT_FORM
+    return cudaGetLastError();
+}
+
+}  // namespace
+
 cudaError_t launch_mover_mixed(const MoverArgs &a, const MixedConsts &c, int sm_count,
                                cudaStream_t s) {
-    if (a.n <= 0) return cudaSuccess;
-    const int threads = 128;
-    const int sp = spread_of(a.ndim, a.n, sm_count);
-    const int64_t blocks = (a.n * sp + threads - 1) / threads;
-    const unsigned g = (unsigned)blocks;
-    const MixedRunArgs r = mixed_run_args(a);
-    if (a.ndim == 2) {
-        if (a.nlgc) mover_mixed_kernel<2, true><<<g, threads, 0, s>>>(r, c, a.P, a.n, sp);
-        else mover_mixed_kernel<2, false><<<g, threads, 0, s>>>(r, c, a.P, a.n, sp);
-    } else {
-        if (a.nlgc) mover_mixed_kernel<3, true><<<g, threads, 0, s>>>(r, c, a.P, a.n, sp);
-        else mover_mixed_kernel<3, false><<<g, threads, 0, s>>>(r, c, a.P, a.n, sp);
-    }
-    return cudaGetLastError();
+    return launch_mover(a, c, nullptr, sm_count, s);
 }
 
 cudaError_t launch_mover_learned(const MoverArgs &a, const MixedConsts &c, const FusedLearn &L,
                                  int sm_count, cudaStream_t s) {
-    if (a.n <= 0) return cudaSuccess;
-    const int sp = spread_of(a.ndim, a.n, sm_count);
-    const unsigned g = (unsigned)((a.n * sp + 127) / 128);
-    const size_t smem = sizeof(mma_mlp::SmemInf);
-    const MixedRunArgs r = mixed_run_args(a);
-    if (a.ndim == 2) {
-        if (a.nlgc) mover_learned_kernel<2, true><<<g, 128, smem, s>>>(r, c, a.P, a.n, sp, L);
-        else mover_learned_kernel<2, false><<<g, 128, smem, s>>>(r, c, a.P, a.n, sp, L);
-    } else {
-        if (a.nlgc) mover_learned_kernel<3, true><<<g, 128, smem, s>>>(r, c, a.P, a.n, sp, L);
-        else mover_learned_kernel<3, false><<<g, 128, smem, s>>>(r, c, a.P, a.n, sp, L);
-    }
-    return cudaGetLastError();
+    return launch_mover(a, c, &L, sm_count, s);
 }
 
 cudaError_t upload_batch_runs(const BatchRun *runs, int nruns, cudaStream_t s) {
@@ -267,25 +286,36 @@ int batch_minb_variants(int ndim, int *out) {
     out[0] = 4; out[1] = 5; return 2;
 }
 
-cudaError_t launch_mover_mixed_batch(int ndim, bool nlgc, int minb, int parity, int nruns,
+cudaError_t launch_mover_mixed_batch(int ndim, bool nlgc, int minb, bool group, int parity, int nruns,
                                      int sm_count, int grab, const long long *tile_prefix,
                                      const unsigned long long *run_n,
                                      unsigned long long *tile_counter,
                                      unsigned long long *nactive_total, cudaStream_t s) {
     const unsigned g = (unsigned)(sm_count * minb);
-#define GPAT_BATCH_LAUNCH(ND, NL, MB)                                                         \
-    mover_mixed_batch_kernel<ND, NL, MB><<<g, 128, 0, s>>>(parity, nruns, tile_prefix, run_n, \
-                                                           tile_counter, grab, nactive_total)
+#define GPAT_BATCH_FORM(ND, NL, MB, GR)                                                           \
+    mover_mixed_batch_kernel<ND, NL, MB, GR><<<g, 128, 0, s>>>(parity, nruns, tile_prefix, run_n, \
+                                                               tile_counter, grab, nactive_total)
+#define GPAT_BATCH_LAUNCH(ND, MB)                                               \
+    do {                                                                        \
+        if (nlgc) {                                                             \
+            if (group) GPAT_BATCH_FORM(ND, true, MB, true);                     \
+            else GPAT_BATCH_FORM(ND, true, MB, false);                          \
+        } else {                                                                \
+            if (group) GPAT_BATCH_FORM(ND, false, MB, true);                    \
+            else GPAT_BATCH_FORM(ND, false, MB, false);                         \
+        }                                                                       \
+    } while (0)
     if (ndim == 2) {
-        if (minb == 5) { if (nlgc) GPAT_BATCH_LAUNCH(2, true, 5); else GPAT_BATCH_LAUNCH(2, false, 5); }
-        else if (minb == 6) { if (nlgc) GPAT_BATCH_LAUNCH(2, true, 6); else GPAT_BATCH_LAUNCH(2, false, 6); }
-        else if (minb == 8) { if (nlgc) GPAT_BATCH_LAUNCH(2, true, 8); else GPAT_BATCH_LAUNCH(2, false, 8); }
+        if (minb == 5) GPAT_BATCH_LAUNCH(2, 5);
+        else if (minb == 6) GPAT_BATCH_LAUNCH(2, 6);
+        else if (minb == 8) GPAT_BATCH_LAUNCH(2, 8);
         else return cudaErrorInvalidValue;
     } else {
-        if (minb == 4) { if (nlgc) GPAT_BATCH_LAUNCH(3, true, 4); else GPAT_BATCH_LAUNCH(3, false, 4); }
-        else if (minb == 5) { if (nlgc) GPAT_BATCH_LAUNCH(3, true, 5); else GPAT_BATCH_LAUNCH(3, false, 5); }
+        if (minb == 4) GPAT_BATCH_LAUNCH(3, 4);
+        else if (minb == 5) GPAT_BATCH_LAUNCH(3, 5);
         else return cudaErrorInvalidValue;
     }
+#undef GPAT_BATCH_FORM
 #undef GPAT_BATCH_LAUNCH
     return cudaGetLastError();
 }
