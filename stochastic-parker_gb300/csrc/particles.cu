@@ -840,7 +840,9 @@ __global__ void __launch_bounds__(kBinScanThreads) bin_tile_scan_kernel(unsigned
 // (2 x 98 B each against 129 MB of L2) the kernel therefore writes only where each
 // particle comes from, and cell_gather_kernel reads the particles in the order in
 // which it writes them: 2e6 particles 254 -> 25 + 155 us, floor 58 us.  Below, one
-// pass: 1e5 particles 14.7 us against 5.7 + 10.5 and a launch.
+// pass: 1e5 particles 14.7 us against 5.7 + 10.5 and a launch.  The list stands in
+// the destination's own rng_ctr, whose entry j the gather reads before it writes
+// particle j.
 constexpr int64_t kGatherFrom = 600000;
 
 // done_key: the trailing done bin (-1: none), whose slots are reserved per
@@ -894,7 +896,7 @@ const unsigned int *cell_sort_counts(const void *scratch, int64_t nbins) {
 
 size_t cell_sort_scratch_bytes(int64_t cap, int64_t nbins) {
     const int64_t ntiles = (nbins + kBinTile - 1) / kBinTile;
-    return (size_t)cap * (cap >= kGatherFrom ? 8 : 4) + (size_t)nbins * 4 + (size_t)(2 * ntiles + 2) * 8 + 256;
+    return (size_t)cap * 4 + (size_t)nbins * 4 + (size_t)(2 * ntiles + 2) * 8 + 256;
 }
 
 cudaError_t launch_cell_sort(const DevParticles &src, const DevParticles &dst, int64_t n,
@@ -910,7 +912,7 @@ cudaError_t launch_cell_sort(const DevParticles &src, const DevParticles &dst, i
     cudaError_t e = cudaMemsetAsync(counts, 0, sizeof(unsigned int) * (size_t)nbins, s);
     if (e != cudaSuccess) return e;
     if (n <= 0) return cudaMemsetAsync(&cnt->nkept, 0, sizeof(unsigned long long), s);
-    uint32_t *from = n >= kGatherFrom ? reinterpret_cast<uint32_t *>(keys + n) : nullptr;
+    uint32_t *from = n >= kGatherFrom ? dst.rng_ctr : nullptr;
     const unsigned blocks = (unsigned)((n + 255) / 256);
     cell_key_kernel<<<blocks, 256, 0, s>>>(src, n, nullptr, g, keys, counts, cnt, esc);
     bin_tile_sum_kernel<<<(unsigned)ntiles, kBinScanThreads, 0, s>>>(counts, nbins, tile_sums);
@@ -935,7 +937,7 @@ cudaError_t launch_cell_sort_dev(const DevParticles &src, const DevParticles &ds
     int32_t *keys = reinterpret_cast<int32_t *>(counts + nbins);
     cudaError_t e = cudaMemsetAsync(counts, 0, sizeof(unsigned int) * (size_t)nbins, s);
     if (e != cudaSuccess) return e;
-    uint32_t *from = cap >= kGatherFrom ? reinterpret_cast<uint32_t *>(keys + cap) : nullptr;
+    uint32_t *from = cap >= kGatherFrom ? dst.rng_ctr : nullptr;
     const unsigned blocks = (unsigned)((cap + 255) / 256);
     if (blocks == 0) return cudaSuccess;
     cell_key_kernel<<<blocks, 256, 0, s>>>(src, 0, n_dev, g, keys, counts, cnt, esc);
