@@ -2167,7 +2167,7 @@ int capture_graphs(gpat_batch_t *b, int nlgc, int minb, int grab) {
             gpat_handle_t *h = b->runs[r];
             e = launch_cell_sort_dev(h->P[parity], h->P[1 - parity], run_n_dev(b) + r, h->cap,
                                      cell_grid(h), h->sort_scratch, h->dcnt, escaped_hist(h),
-                                     b->stream);
+                                     b->sm_count, b->stream);
         }
         cudaGraph_t g = nullptr;
         const cudaError_t ee = cudaStreamEndCapture(b->stream, &g);

@@ -284,7 +284,7 @@ struct CellGrid;
 struct EscHist;
 cudaError_t launch_cell_sort_dev(const DevParticles &src, const DevParticles &dst,
                                  unsigned long long *n_dev, int64_t cap, const CellGrid &g,
-                                 void *scratch, DevCounters *cnt, const EscHist &esc,
+                                 void *scratch, DevCounters *cnt, const EscHist &esc, int sm_count,
                                  cudaStream_t s);
 cudaError_t launch_mover_mixed_batch(int ndim, bool nlgc, int minb, bool group, int parity, int nruns,
                                      int sm_count, int grab, const long long *tile_prefix,

@@ -847,7 +847,8 @@ constexpr int64_t kGatherFrom = 600000;
 
 // done_key: the trailing done bin (-1: none), whose slots are reserved per
 // warp, one atomic for all its lanes that go there.  from: the index list, or
-// null to move the particles themselves.
+// null (and, where the count stands on the device, below kGatherFrom) to move the
+// particles themselves.
 __global__ void __launch_bounds__(256) cell_scatter_kernel(const DevParticles S, const DevParticles D,
                                                            int64_t n,
                                                            const unsigned long long *n_dev,
@@ -856,6 +857,7 @@ __global__ void __launch_bounds__(256) cell_scatter_kernel(const DevParticles S,
                                                            uint32_t *from) {
     const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (n_dev) n = (int64_t)*n_dev;
+    if (n < kGatherFrom) from = nullptr;
     const int32_t key = i < n ? keys[i] : -1;
     const unsigned dm = __ballot_sync(0xffffffffu, key >= 0 && key == done_key);
     unsigned int pos = 0;
@@ -873,11 +875,16 @@ __global__ void __launch_bounds__(256) cell_scatter_kernel(const DevParticles S,
     else copy_particle(S, i, D, (int64_t)pos);
 }
 
+// n_dev: the scatter's count where it stands on the device; nothing to do below
+// kGatherFrom.
 __global__ void __launch_bounds__(256) cell_gather_kernel(const DevParticles S, const DevParticles D,
+                                                          const unsigned long long *n_dev,
                                                           const unsigned long long *nkept,
                                                           const uint32_t *from) {
-    const int64_t j = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (j < (int64_t)*nkept) copy_particle(S, (int64_t)from[j], D, j);
+    if (n_dev && (int64_t)*n_dev < kGatherFrom) return;
+    const int64_t kept = (int64_t)*nkept, stride = (int64_t)gridDim.x * blockDim.x;
+    for (int64_t j = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; j < kept; j += stride)
+        copy_particle(S, (int64_t)from[j], D, j);
 }
 
 }  // namespace
@@ -920,13 +927,13 @@ cudaError_t launch_cell_sort(const DevParticles &src, const DevParticles &dst, i
     bin_tile_scan_kernel<<<(unsigned)ntiles, kBinScanThreads, 0, s>>>(counts, nbins, tile_offsets);
     cell_scatter_kernel<<<blocks, 256, 0, s>>>(src, dst, n, nullptr, keys, counts,
                                                g.done_bin ? (int32_t)(nbins - 1) : -1, from);
-    if (from) cell_gather_kernel<<<blocks, 256, 0, s>>>(src, dst, &cnt->nkept, from);
+    if (from) cell_gather_kernel<<<blocks, 256, 0, s>>>(src, dst, nullptr, &cnt->nkept, from);
     return cudaGetLastError();
 }
 
 cudaError_t launch_cell_sort_dev(const DevParticles &src, const DevParticles &dst,
                                  unsigned long long *n_dev, int64_t cap, const CellGrid &g,
-                                 void *scratch, DevCounters *cnt, const EscHist &esc,
+                                 void *scratch, DevCounters *cnt, const EscHist &esc, int sm_count,
                                  cudaStream_t s) {
     const int64_t nbins = cell_grid_bins(g);
     const int64_t ntiles = (nbins + kBinTile - 1) / kBinTile;
@@ -946,7 +953,10 @@ cudaError_t launch_cell_sort_dev(const DevParticles &src, const DevParticles &ds
     bin_tile_scan_kernel<<<(unsigned)ntiles, kBinScanThreads, 0, s>>>(counts, nbins, tile_offsets);
     cell_scatter_kernel<<<blocks, 256, 0, s>>>(src, dst, 0, n_dev, keys, counts,
                                                g.done_bin ? (int32_t)(nbins - 1) : -1, from);
-    if (from) cell_gather_kernel<<<blocks, 256, 0, s>>>(src, dst, &cnt->nkept, from);
+    // of a size that costs little where the run has few particles for its capacity
+    if (from)
+        cell_gather_kernel<<<std::min(blocks, 8u * (unsigned)sm_count), 256, 0, s>>>(
+            src, dst, n_dev, &cnt->nkept, from);
     e = cudaGetLastError();
     if (e != cudaSuccess) return e;
     return cudaMemcpyAsync(n_dev, &cnt->nkept, sizeof(unsigned long long),
