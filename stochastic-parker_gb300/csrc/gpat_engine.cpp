@@ -72,9 +72,6 @@ struct gpat_handle {
     // distributions: bins, then weights and counts on their way to the host
     unsigned long long *bins_ws = nullptr;
     size_t bins_ws_bytes = 0;
-    // FP64 mover: the order its lanes take the particles in
-    uint32_t *work = nullptr;
-    int64_t work_cap = 0;
     // learned splitting inside the mover (gpat_set_mover_learned): the
     // launch arguments, and on the device the particle count with children,
     // the judged count and the fixed-point sum of w exp(z - z_shift)
@@ -762,7 +759,6 @@ int gpat_destroy(gpat_handle_t *h) {
     if (h->sort_scratch) cudaFree(h->sort_scratch);
     if (h->tile_dev) cudaFree(h->tile_dev);
     if (h->pause) cudaFree(h->pause);
-    if (h->work) cudaFree(h->work);
     if (h->bins_ws) cudaFree(h->bins_ws);
     if (h->learn_dev) cudaFree(h->learn_dev);
     if (h->fresh_dev) cudaFree(h->fresh_dev);
@@ -1626,19 +1622,10 @@ int gpat_particle_mover(gpat_handle_t *h, int focused_transport, int nlgc, doubl
         }
     } else {
         if (mover_fp64_orders(h->n, h->sm_count)) {
-            if (h->n > h->work_cap) {
-                CK(cudaStreamSynchronize(h->stream));
-                if (h->work) CK(cudaFree(h->work));
-                h->work = nullptr;
-                h->work_cap = 0;
-                if (cudaMalloc(&h->work, sizeof(uint32_t) * ((size_t)h->cap + kOrderHead)) !=
-                    cudaSuccess) {
-                    cudaGetLastError();
-                    return fail(h, GPAT_ERR_OOM, "work list");
-                }
-                h->work_cap = h->cap;
-            }
-            a.work = h->work;
+            // in the other buffer, which nothing reads before the removal writes it
+            const DevParticles &spare = h->P[1 - h->cur];
+            a.work = spare.rng_ctr;
+            a.work_head = reinterpret_cast<uint32_t *>(spare.tag_splitted);
         }
         CK(cudaEventRecord(h->ev0, h->stream));
         CK(launch_mover_fp64(a, h->sm_count, h->stream));

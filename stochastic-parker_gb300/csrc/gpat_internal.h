@@ -132,10 +132,10 @@ struct MoverArgs {
     double rdx, rdy, rdz, rdtf, rp0, d1p0, d2p0sq, sdt_min, sdt_max;
     int drift_finite;   // the drift's prefactor is finite for any momentum
     // FP64 mover's work list: lanes of a warp that take particles, and the
-    // order they are taken in (kOrderHead words of scratch, then the indices;
-    // null: by index).
+    // order they are taken in (null: by index), with kOrderHead words of scratch
+    // for making it.
     int lanes;
-    uint32_t *work;
+    uint32_t *work, *work_head;
 };
 
 // Single-precision constants of the split-precision mover, derived on the
@@ -258,8 +258,7 @@ cudaError_t launch_mover_fp64(const MoverArgs &a, int sm_count, cudaStream_t s);
 // The same in teams of kMoverTeam lanes, for launch_mover_fp64.
 constexpr int kMoverTeam = 8;
 cudaError_t launch_mover_fp64_team(const MoverArgs &a, int sm_count, cudaStream_t s);
-// Whether that launch orders n particles, for which MoverArgs::work has room
-// for kOrderHead + n words.
+// Whether that launch orders n particles, for which MoverArgs::work has n words.
 constexpr int kOrderHead = 128;
 bool mover_fp64_orders(int64_t n, int sm_count);
 cudaError_t launch_mover_mixed(const MoverArgs &a, const MixedConsts &c, int sm_count,

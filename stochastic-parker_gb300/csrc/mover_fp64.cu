@@ -1609,7 +1609,7 @@ __global__ void __launch_bounds__(128) mover_fp64_kernel(const MoverArgs a) {
             if (have || !taker) continue;
             i = (int64_t)(base + __popc(need & ((1u << lane) - 1u)));
             if (i >= a.n) continue;
-            if (a.work) i = (int64_t)a.work[kOrderHead + i];
+            if (a.work) i = (int64_t)a.work[i];
             have = true;
             s.x = a.P.x[i]; s.y = a.P.y[i]; s.z = a.P.z[i]; s.p = a.P.p[i];
             s.v = FT ? a.P.v[i] : 0.0;
@@ -1758,7 +1758,7 @@ __global__ void __launch_bounds__(256) order_count_kernel(const MoverArgs a, flo
         atomicAdd(&bins[order_bin(a, i, step0)], 1u);
     __syncthreads();
     if (threadIdx.x < kOrderBins && bins[threadIdx.x])
-        atomicAdd(&a.work[threadIdx.x], bins[threadIdx.x]);
+        atomicAdd(&a.work_head[threadIdx.x], bins[threadIdx.x]);
 }
 
 __global__ void __launch_bounds__(256) order_scatter_kernel(const MoverArgs a, float step0) {
@@ -1775,11 +1775,12 @@ __global__ void __launch_bounds__(256) order_scatter_kernel(const MoverArgs a, f
     __syncthreads();
     if (threadIdx.x < kOrderBins && bins[threadIdx.x]) {
         uint32_t first = 0;
-        for (int k = 0; k < threadIdx.x; ++k) first += a.work[k];
-        base[threadIdx.x] = first + atomicAdd(&a.work[kOrderBins + threadIdx.x], bins[threadIdx.x]);
+        for (int k = 0; k < threadIdx.x; ++k) first += a.work_head[k];
+        base[threadIdx.x] =
+            first + atomicAdd(&a.work_head[kOrderBins + threadIdx.x], bins[threadIdx.x]);
     }
     __syncthreads();
-    if (i < a.n) a.work[kOrderHead + base[b] + rank] = (uint32_t)i;
+    if (i < a.n) a.work[base[b] + rank] = (uint32_t)i;
 }
 
 #endif
@@ -1823,7 +1824,7 @@ cudaError_t launch_mover_fp64_team(const MoverArgs &args, int sm_count, cudaStre
     if (e != cudaSuccess) return e;
 #if GPAT_FP64_TEAM == 1
     if (a.work) {
-        e = cudaMemsetAsync(a.work, 0, sizeof(uint32_t) * kOrderHead, s);
+        e = cudaMemsetAsync(a.work_head, 0, sizeof(uint32_t) * kOrderHead, s);
         if (e != cudaSuccess) return e;
         double h = a.dx;
         if (!a.spherical && a.ndim > 1) h = std::min(h, a.dy);

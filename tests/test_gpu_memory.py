@@ -49,3 +49,22 @@ def test_bytes_per_particle_of_the_split_precision_mover():
     taken = free - torch.cuda.mem_get_info(0)[0]
     eng.close()
     assert taken <= cap * (2 * 98 + 4 + 1) + (24 << 20), taken / cap
+
+
+def test_bytes_per_particle_of_the_fp64_mover():
+    """Two sets of 98 bytes, through a call that orders its particles."""
+    cap, n = 30_000_000, 100_000
+    _taken(2, 16, 1)
+    cfg = make_mhd_config(32, 32, 1, 0.0, 1.0, 0.0, 1.0, dt_out=1e-3)
+    prm = make_params(ndim=2, p0=0.1, pmin=0.1, pmax=1.0, kpara0=1e-3, dt_min_rel=0.1, dt_max_rel=0.5,
+                      nptl_max=cap, seed=3, precision=0)
+    free = torch.cuda.mem_get_info(0)[0]
+    eng = Engine(prm, cfg, 0)
+    eng.set_tstamps(np.arange(3) * 1e-3)
+    eng.set_fields(fields.planar_shock_2d(32, 32, 0.0, 1.0, 0.0, 1.0, r=3.0, w=0.05, x0=0.5), 0)
+    eng.calc_fields_gradients(0)
+    eng.inject_particles_spatial_uniform(n, 1e-6, 2, 1.0, 1, (0.0, 0.0, 0.0, 1.0, 1.0, 1.0), 1.0)
+    eng.particle_mover(mhd_tframe=1)
+    taken = free - torch.cuda.mem_get_info(0)[0]
+    eng.close()
+    assert taken <= cap * 2 * 98 + (24 << 20), taken / cap
