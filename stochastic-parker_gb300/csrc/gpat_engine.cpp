@@ -263,6 +263,20 @@ struct ConfScanner {
 
 int to_int_via_real4(double v) { return (int)(float)v; }
 
+// Behind a slot's packed records and behind its fluctuation records: the word that
+// says whether some value of them is subnormal, infinite or NaN.  It is copied with
+// them.
+constexpr size_t kFrameTail = 4;   // floats
+
+unsigned int *odd_fields(const gpat_handle_t *h, int slot) {
+    const size_t R = (h->prm.ndim == 2) ? kRec2D : kRec3D;
+    return reinterpret_cast<unsigned int *>(h->rec[slot] + R * h->ncells);
+}
+
+unsigned int *odd_aux(const gpat_handle_t *h, int slot) {
+    return reinterpret_cast<unsigned int *>(h->aux[slot] + 16 * h->ncells);
+}
+
 int mover_args(gpat_handle_t *h, int mhd_tframe, int nsteps_interval, int num_fine_steps,
                MoverArgs &a) {
     const gpat_params_t &p = h->prm;
@@ -284,6 +298,11 @@ int mover_args(gpat_handle_t *h, int mhd_tframe, int nsteps_interval, int num_fi
     a.correlation_flag = p.correlation_flag;
     a.aux1 = h->aux[0];
     a.aux2 = p.time_interp ? h->aux[1] : h->aux[0];
+    const int second = p.time_interp ? 1 : 0;
+    a.odd1 = odd_fields(h, 0);
+    a.odd2 = odd_fields(h, second);
+    if (h->aux[0]) a.odd_aux1 = odd_aux(h, 0);
+    if (h->aux[second]) a.odd_aux2 = odd_aux(h, second);
     a.duu0 = p.duu0;
     a.dpp_wave = p.dpp_wave;
     a.dpp_shear = p.dpp_shear;
@@ -677,15 +696,16 @@ int gpat_create(const gpat_params_t *params, const gpat_mhd_config_t *cfg, int d
     const int R = (p.ndim == 2) ? kRec2D : kRec3D;
     for (int s = 0; s < h->nslots; ++s) {
         if (cudaMalloc(&h->full[s], 32 * sizeof(float) * h->ncells) != cudaSuccess ||
-            cudaMalloc(&h->rec[s], (size_t)R * sizeof(float) * h->ncells) != cudaSuccess)
+            cudaMalloc(&h->rec[s], sizeof(float) * ((size_t)R * h->ncells + kFrameTail)) != cudaSuccess)
             return bail(GPAT_ERR_OOM);
         cudaMemsetAsync(h->full[s], 0, 32 * sizeof(float) * h->ncells, h->stream);
         // init_magnetic_fluctuation / init_correlation_length
         // (mhd_data_parallel.f90:107-182): every component starts at 1
         if (p.deltab_flag || p.correlation_flag) {
-            if (cudaMalloc(&h->aux[s], 16 * sizeof(float) * h->ncells) != cudaSuccess)
+            if (cudaMalloc(&h->aux[s], sizeof(float) * (16 * h->ncells + kFrameTail)) != cudaSuccess)
                 return bail(GPAT_ERR_OOM);
-            if (launch_fill(h->aux[s], 1.0f, 16 * h->ncells, h->stream) != cudaSuccess)
+            if (launch_fill(h->aux[s], 1.0f, 16 * h->ncells, h->stream) != cudaSuccess ||
+                cudaMemsetAsync(odd_aux(h, s), 0, sizeof(unsigned int), h->stream) != cudaSuccess)
                 return bail(GPAT_ERR_CUDA);
         }
     }
@@ -826,7 +846,7 @@ int gpat_set_fields(gpat_handle_t *h, int var_flag, const float *farray, int nva
         CK(cudaMemcpyAsync(h->full[slot], farray, 32 * sizeof(float) * h->ncells,
                            cudaMemcpyHostToDevice, h->stream));
         CK(launch_pack_records(h->full[slot], h->rec[slot], h->prm.ndim, h->ncells,
-                               &h->dcnt->odd_fields[slot], h->stream));
+                               odd_fields(h, slot), h->stream));
         h->rec_ready[slot] = true;
         ++h->rec_gen[slot];
     } else {
@@ -869,7 +889,7 @@ int gpat_set_fluctuations(gpat_handle_t *h, int var_flag, const float *db2_slab,
     const gpat_mhd_config_t &c = h->cfg;
     CK(launch_calc_aux_gradients(h->aux[slot], h->prm.ndim, h->nxg, h->nyg, h->nzg, c.dx, c.dy,
                                  c.dz, h->stream, grad_spans(h)));
-    CK(launch_find_odd(h->aux[slot], 16 * h->ncells, &h->dcnt->odd_aux[slot], h->stream));
+    CK(launch_find_odd(h->aux[slot], 16 * h->ncells, odd_aux(h, slot), h->stream));
     CK(cudaStreamSynchronize(h->stream));
     return GPAT_OK;
 }
@@ -1061,8 +1081,7 @@ int gpat_calc_fields_gradients(gpat_handle_t *h, int var_flag) {
     CK(cudaSetDevice(h->device));
     const gpat_mhd_config_t &c = h->cfg;
     CK(launch_calc_fields_gradients(h->full[slot], h->rec[slot], h->prm.ndim, h->nxg, h->nyg, h->nzg,
-                                    c.dx, c.dy, c.dz, grad_spans(h), &h->dcnt->odd_fields[slot],
-                                    h->stream));
+                                    c.dx, c.dy, c.dz, grad_spans(h), odd_fields(h, slot), h->stream));
     CK(cudaStreamSynchronize(h->stream));
     h->rec_ready[slot] = true;
     ++h->rec_gen[slot];
@@ -1076,14 +1095,10 @@ int gpat_copy_fields(gpat_handle_t *h) {
     const int R = (h->prm.ndim == 2) ? kRec2D : kRec3D;
     CK(cudaMemcpyAsync(h->full[0], h->full[1], 32 * sizeof(float) * h->ncells,
                        cudaMemcpyDeviceToDevice, h->stream));
-    CK(cudaMemcpyAsync(h->rec[0], h->rec[1], (size_t)R * sizeof(float) * h->ncells,
-                       cudaMemcpyDeviceToDevice, h->stream));
-    CK(cudaMemcpyAsync(&h->dcnt->odd_fields[0], &h->dcnt->odd_fields[1], sizeof(unsigned int),
-                       cudaMemcpyDeviceToDevice, h->stream));
-    CK(cudaMemcpyAsync(&h->dcnt->odd_aux[0], &h->dcnt->odd_aux[1], sizeof(unsigned int),
+    CK(cudaMemcpyAsync(h->rec[0], h->rec[1], sizeof(float) * ((size_t)R * h->ncells + kFrameTail),
                        cudaMemcpyDeviceToDevice, h->stream));
     if (h->aux[0] && h->aux[1])   // copy_magnetic_fluctuation / copy_correlation_length
-        CK(cudaMemcpyAsync(h->aux[0], h->aux[1], 16 * sizeof(float) * h->ncells,
+        CK(cudaMemcpyAsync(h->aux[0], h->aux[1], sizeof(float) * (16 * h->ncells + kFrameTail),
                            cudaMemcpyDeviceToDevice, h->stream));
     for (int k = 0; k < 2; ++k)   // copy_acc_surface
         if (h->dsurf[k][0] && h->dsurf[k][1])

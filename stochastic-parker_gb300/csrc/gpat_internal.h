@@ -51,9 +51,6 @@ struct DevCounters {
     unsigned long long trk_dropped;  // tracked records past nsteps_tracking_max
     unsigned long long pmax_bits;    // get_pmax_global: bits of the largest p >= 0
     unsigned long long next;         // FP64 mover launch: particles handed out so far
-    // per frame slot: some field value (or fluctuation value) is subnormal,
-    // infinite or NaN
-    unsigned int odd_fields[2], odd_aux[2];
     unsigned int tag_top, tag_low;   // launch_tag_range
 };
 
@@ -131,6 +128,9 @@ struct MoverArgs {
     // the products and roots of the run's constants that every push needs.
     double rdx, rdy, rdz, rdtf, rp0, d1p0, d2p0sq, sdt_min, sdt_max;
     int drift_finite;   // the drift's prefactor is finite for any momentum
+    // FP64 mover, per frame: whether some field (fluctuation) value is subnormal,
+    // infinite or NaN.
+    const unsigned int *odd1, *odd2, *odd_aux1, *odd_aux2;
     // FP64 mover's work list: lanes of a warp that take particles, and the
     // order they are taken in (null: by index), with kOrderHead words of scratch
     // for making it.

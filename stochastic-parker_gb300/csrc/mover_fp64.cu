@@ -129,11 +129,11 @@ __device__ __forceinline__ bool uniform_cell(const MoverArgs &a, const State &s,
 
 // NV variables of records of R floats interpolated with corner (ix, iy, iz)
 // and weights w, time-interpolated between the two frames; odd: per frame, a
-// value that needs the plain product (DevCounters::odd_fields, odd_aux).
+// value that needs the plain product (MoverArgs::odd1, odd_aux1).
 template <int NDIM, int NV, int R>
 __device__ __forceinline__ void interp_at(const MoverArgs &a, const float *rec1, const float *rec2,
-                                          const unsigned int *odd, const State &s, int ix, int iy,
-                                          int iz, const double *w, double f[NV]) {
+                                          const unsigned int *odd1, const unsigned int *odd2,
+                                          const State &s, int ix, int iy, int iz, const double *w, double f[NV]) {
     // One copy of the code for both frames and, but for the first, for all
     // corners: unrolled over them it does not fit the instruction cache, and
     // with one warp per scheduler every miss is waited for.
@@ -143,7 +143,7 @@ __device__ __forceinline__ void interp_at(const MoverArgs &a, const float *rec1,
 #pragma unroll 1
     for (int frame = a.time_interp ? 1 : 0; frame >= 0; --frame) {
         const float *rec = (frame ? rec2 : rec1) + (size_t)R * cell;
-        const bool plain = __ldg(odd + (a.time_interp ? frame : 0)) != 0u;
+        const bool plain = __ldg(frame ? odd2 : odd1) != 0u;
         add_corner<NV, true>(rec, w[0], plain, f);
 #pragma unroll 1
         for (int c = 1; c < kCorners; ++c) {
@@ -171,7 +171,8 @@ __device__ __forceinline__ void interp_at(const MoverArgs &a, const float *rec1,
 // lanes of the warp call; want: the first lane's particle makes a push.
 template <int NDIM, int NV, int R>
 __device__ __forceinline__ void interp_team(const MoverArgs &a, const float *rec1,
-                                            const float *rec2, const unsigned int *odd,
+                                            const float *rec2, const unsigned int *odd1,
+                                            const unsigned int *odd2,
                                             const State &s, bool want, int ix, int iy, int iz,
                                             const double *w, double f[NV]) {
     constexpr int kCorners = NDIM == 3 ? 8 : NDIM == 2 ? 4 : 2;
@@ -190,7 +191,7 @@ __device__ __forceinline__ void interp_team(const MoverArgs &a, const float *rec
 #pragma unroll 1
     for (int frame = a.time_interp ? 1 : 0; frame >= 0; --frame) {
         const float *rec = (frame ? rec2 : rec1) + (size_t)R * cell + sub;
-        const bool plain = __ldg(odd + (a.time_interp ? frame : 0)) != 0u;
+        const bool plain = __ldg(frame ? odd2 : odd1) != 0u;
 #pragma unroll
         for (int c = 0; c < kCorners; ++c) {
             size_t off = (size_t)(c & 1);
@@ -229,11 +230,12 @@ __device__ __forceinline__ void interp_team(const MoverArgs &a, const float *rec
 
 template <int NDIM, int NV, int R>
 __device__ __forceinline__ void interpolate(const MoverArgs &a, const float *rec1,
-                                            const float *rec2, const unsigned int *odd,
+                                            const float *rec2, const unsigned int *odd1,
+                                            const unsigned int *odd2,
                                             const State &s, bool want, int ix, int iy, int iz,
                                             const double *w, double f[NV]) {
-    if (kTeam > 1) interp_team<NDIM, NV, R>(a, rec1, rec2, odd, s, want, ix, iy, iz, w, f);
-    else if (want) interp_at<NDIM, NV, R>(a, rec1, rec2, odd, s, ix, iy, iz, w, f);
+    if (kTeam > 1) interp_team<NDIM, NV, R>(a, rec1, rec2, odd1, odd2, s, want, ix, iy, iz, w, f);
+    else if (want) interp_at<NDIM, NV, R>(a, rec1, rec2, odd1, odd2, s, ix, iy, iz, w, f);
 }
 
 // Field values at the particle under the reference's names.
@@ -1511,19 +1513,18 @@ __device__ __forceinline__ bool do_push(const MoverArgs &a, State &s, bool want,
     const double *aux = nullptr;
     if (FULL || GRID) {
         double v[32];
-        interpolate<NDIM, 32, 32>(a, a.full1, a.full2, a.cnt->odd_fields, s, ok, c.ix, c.iy, c.iz,
-                                  c.w, v);
+        interpolate<NDIM, 32, 32>(a, a.full1, a.full2, a.odd1, a.odd2, s, ok, c.ix, c.iy, c.iz, c.w, v);
         f = named_full(v);
         if (a.aux1 && (a.deltab_flag || a.correlation_flag)) {
-            interpolate<NDIM, 16, 16>(a, a.aux1, a.aux2, a.cnt->odd_aux, s, ok, c.ix, c.iy, c.iz,
-                                      c.w, av);
+            interpolate<NDIM, 16, 16>(a, a.aux1, a.aux2, a.odd_aux1, a.odd_aux2, s, ok, c.ix,
+                                      c.iy, c.iz, c.w, av);
             aux = av;
         }
     } else {
         constexpr int NV = (NDIM == 2) ? 15 : 21;
         constexpr int R = (NDIM == 2) ? kRec2D : kRec3D;
         double v[NV];
-        interpolate<NDIM, NV, R>(a, a.rec1, a.rec2, a.cnt->odd_fields, s, ok, c.ix, c.iy, c.iz, c.w,
+        interpolate<NDIM, NV, R>(a, a.rec1, a.rec2, a.odd1, a.odd2, s, ok, c.ix, c.iy, c.iz, c.w,
                                  v);
         f = named_packed<NDIM>(v);
     }
