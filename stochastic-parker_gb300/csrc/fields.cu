@@ -49,51 +49,59 @@ __device__ __forceinline__ float grad_c(float ap, float am, double ih) {
     return (float)__dmul_rn((double)__fsub_rn(ap, am), ih);
 }
 
-// Gradients of NVAR variables of records of STRIDE floats (value of v at
-// v * VSTRIDE, its d/dx d/dy d/dz at GBASE + v * GSTEP + axis); the z
-// component only in 3D.  <32, 8, 1, 8, 3>: the field records; <16, 4, 4, 1, 4>:
-// the fluctuation records {db2_slab, db2_2d, lc_slab, lc_2d}.  ihx/ihy/ihz:
-// per-node inverse spans of a non-uniform grid (idxh_grid of
+// Gradients of the fluctuation records {db2_slab, db2_2d, lc_slab, lc_2d}, 16 floats
+// a node: value v at 4 v, its d/dx d/dy d/dz behind it; the z component only in 3D.
+// ihx/ihy/ihz: per-node inverse spans of a non-uniform grid (idxh_grid of
 // set_local_grid_positions, mhd_data_parallel.f90:2153-2190, as used by
-// calc_fields_gradients_nonuniform :612-764), or null for 0.5 / d.
-template <int STRIDE, int NVAR, int VSTRIDE, int GBASE, int GSTEP>
-__global__ void gradients_kernel(float *__restrict__ a, int ndim, int nxg, int nyg, int nzg,
-                                 double idxh, double idyh, double idzh,
-                                 const double *__restrict__ ihx, const double *__restrict__ ihy,
-                                 const double *__restrict__ ihz) {
+// calc_fields_gradients_nonuniform :612-764), or null for 0.5 / d.  odd_found: set
+// where a value or a gradient is subnormal, infinite or NaN; the values are looked
+// at where the x differences have read them, node i + 1 at node i.
+__global__ void aux_gradients_kernel(float *__restrict__ a, int ndim, int nxg, int nyg, int nzg,
+                                     double idxh, double idyh, double idzh,
+                                     const double *__restrict__ ihx, const double *__restrict__ ihy,
+                                     const double *__restrict__ ihz, unsigned int *odd_found) {
     const size_t ncells = (size_t)nxg * nyg * nzg;
     const size_t stride = (size_t)gridDim.x * blockDim.x;
-    const size_t sx = STRIDE, sy = STRIDE * (size_t)nxg, sz = STRIDE * (size_t)nxg * nyg;
+    const size_t sx = 16, sy = 16 * (size_t)nxg, sz = 16 * (size_t)nxg * nyg;
+    bool odd = false;
     for (size_t c = (size_t)blockIdx.x * blockDim.x + threadIdx.x; c < ncells; c += stride) {
         const int i = (int)(c % nxg);
         const int j = (int)((c / nxg) % nyg);
         const int k = (int)(c / ((size_t)nxg * nyg));
-        float *cell = a + STRIDE * c;
         const double hx = ihx ? ihx[i] : idxh;
         const double hy = ihy ? ihy[j] : idyh;
         const double hz = ihz ? ihz[k] : idzh;
 #pragma unroll
-        for (int v = 0; v < NVAR; ++v) {
-            const int x = v * VSTRIDE, g = GBASE + v * GSTEP;
-            float d;
-            if (i == 0) d = grad_lo(cell[x], cell[x + sx], cell[x + 2 * sx], hx);
-            else if (i == nxg - 1) d = grad_hi(cell[x], cell[x - sx], cell[x - 2 * sx], hx);
-            else d = grad_c(cell[x + sx], cell[x - sx], hx);
-            cell[g] = d;
+        for (int v = 0; v < 4; ++v) {
+            float *cell = a + 16 * c + 4 * v, d;
+            if (i == 0) {
+                d = grad_lo(cell[0], cell[sx], cell[2 * sx], hx);
+                odd |= odd_float(cell[0]) | odd_float(cell[sx]);
+            } else if (i == nxg - 1) {
+                d = grad_hi(cell[0], *(cell - sx), *(cell - 2 * sx), hx);
+            } else {
+                d = grad_c(cell[sx], *(cell - sx), hx);
+                odd |= odd_float(cell[sx]);
+            }
+            cell[1] = d;
+            odd |= odd_float(d);
             if (nyg > 1) {
-                if (j == 0) d = grad_lo(cell[x], cell[x + sy], cell[x + 2 * sy], hy);
-                else if (j == nyg - 1) d = grad_hi(cell[x], cell[x - sy], cell[x - 2 * sy], hy);
-                else d = grad_c(cell[x + sy], cell[x - sy], hy);
-                cell[g + 1] = d;
+                if (j == 0) d = grad_lo(cell[0], cell[sy], cell[2 * sy], hy);
+                else if (j == nyg - 1) d = grad_hi(cell[0], *(cell - sy), *(cell - 2 * sy), hy);
+                else d = grad_c(cell[sy], *(cell - sy), hy);
+                cell[2] = d;
+                odd |= odd_float(d);
             }
             if (nzg > 1 && ndim == 3) {
-                if (k == 0) d = grad_lo(cell[x], cell[x + sz], cell[x + 2 * sz], hz);
-                else if (k == nzg - 1) d = grad_hi(cell[x], cell[x - sz], cell[x - 2 * sz], hz);
-                else d = grad_c(cell[x + sz], cell[x - sz], hz);
-                cell[g + 2] = d;
+                if (k == 0) d = grad_lo(cell[0], cell[sz], cell[2 * sz], hz);
+                else if (k == nzg - 1) d = grad_hi(cell[0], *(cell - sz), *(cell - 2 * sz), hz);
+                else d = grad_c(cell[sz], *(cell - sz), hz);
+                cell[3] = d;
+                odd |= odd_float(d);
             }
         }
     }
+    if (odd) *odd_found = 1u;
 }
 
 // (float)((double)t * ih), the reference's rounding to double and then to
@@ -234,14 +242,16 @@ cudaError_t launch_pack_records(const float *full, float *rec, int ndim, size_t 
 
 cudaError_t launch_calc_aux_gradients(float *aux, int ndim, int nxg, int nyg, int nzg, double dx,
                                       double dy, double dz, cudaStream_t s,
-                                      const double *const *ih) {
+                                      const double *const *ih, unsigned int *odd) {
+    const cudaError_t e = cudaMemsetAsync(odd, 0, sizeof(unsigned int), s);
+    if (e != cudaSuccess) return e;
     const size_t ncells = (size_t)nxg * nyg * nzg;
     const int threads = 256;
     size_t blocks = (ncells + threads - 1) / threads;
     if (blocks > 65535 * 16) blocks = 65535 * 16;
-    gradients_kernel<16, 4, 4, 1, 4><<<(unsigned)blocks, threads, 0, s>>>(
+    aux_gradients_kernel<<<(unsigned)blocks, threads, 0, s>>>(
         aux, ndim, nxg, nyg, nzg, 0.5 / dx, 0.5 / dy, 0.5 / dz, ih ? ih[0] : nullptr,
-        ih ? ih[1] : nullptr, ih ? ih[2] : nullptr);
+        ih ? ih[1] : nullptr, ih ? ih[2] : nullptr, odd);
     return cudaGetLastError();
 }
 
@@ -274,22 +284,6 @@ cudaError_t launch_fill(float *a, float v, size_t n, cudaStream_t s) {
     if (blocks > 65535 * 16) blocks = 65535 * 16;
     if (blocks == 0) return cudaSuccess;
     fill_kernel<<<(unsigned)blocks, threads, 0, s>>>(a, v, n);
-    return cudaGetLastError();
-}
-
-__global__ void find_odd_kernel(const float *__restrict__ a, size_t n, unsigned int *odd_found) {
-    const size_t stride = (size_t)gridDim.x * blockDim.x;
-    bool odd = false;
-    for (size_t c = (size_t)blockIdx.x * blockDim.x + threadIdx.x; c < n; c += stride)
-        odd |= odd_float(a[c]);
-    if (odd) *odd_found = 1u;
-}
-
-cudaError_t launch_find_odd(const float *a, size_t n, unsigned int *odd, cudaStream_t s) {
-    const cudaError_t e = cudaMemsetAsync(odd, 0, sizeof(unsigned int), s);
-    if (e != cudaSuccess || n == 0) return e;
-    const size_t blocks = (n + 255) / 256;
-    find_odd_kernel<<<(unsigned)(blocks < 65535 ? blocks : 65535), 256, 0, s>>>(a, n, odd);
     return cudaGetLastError();
 }
 

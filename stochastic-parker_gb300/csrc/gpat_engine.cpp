@@ -888,8 +888,7 @@ int gpat_set_fluctuations(gpat_handle_t *h, int var_flag, const float *db2_slab,
     }
     const gpat_mhd_config_t &c = h->cfg;
     CK(launch_calc_aux_gradients(h->aux[slot], h->prm.ndim, h->nxg, h->nyg, h->nzg, c.dx, c.dy,
-                                 c.dz, h->stream, grad_spans(h)));
-    CK(launch_find_odd(h->aux[slot], 16 * h->ncells, odd_aux(h, slot), h->stream));
+                                 c.dz, h->stream, grad_spans(h), odd_aux(h, slot)));
     CK(cudaStreamSynchronize(h->stream));
     return GPAT_OK;
 }

@@ -237,8 +237,6 @@ cudaError_t launch_calc_fields_gradients(float *full, float *rec, int ndim, int 
 // The packed records alone (frames that come with their gradients); odd as above.
 cudaError_t launch_pack_records(const float *full, float *rec, int ndim, size_t ncells,
                                 unsigned int *odd, cudaStream_t s);
-// The same over n floats.
-cudaError_t launch_find_odd(const float *a, size_t n, unsigned int *odd, cudaStream_t s);
 // Chunk-planar copy of packed records (planes of float4, one per 16-byte chunk
 // of the record that holds data) for the tile mover.
 cudaError_t launch_planarize_records(const float *rec, float *planes, int ndim, size_t ncells,
@@ -247,7 +245,7 @@ cudaError_t launch_planarize_records(const float *rec, float *planes, int ndim, 
 // lc_2d} x {value, d/dx, d/dy, d/dz}.
 cudaError_t launch_calc_aux_gradients(float *aux, int ndim, int nxg, int nyg, int nzg, double dx,
                                       double dy, double dz, cudaStream_t s,
-                                      const double *const *ih = nullptr);
+                                      const double *const *ih, unsigned int *odd);
 cudaError_t launch_scatter_aux(const float *src, float *aux, int comp, size_t ncells,
                                cudaStream_t s);
 cudaError_t launch_fill(float *a, float v, size_t n, cudaStream_t s);
