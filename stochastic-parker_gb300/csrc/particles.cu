@@ -1227,6 +1227,25 @@ __global__ void __launch_bounds__(256) local_dist_kernel(const DevParticles P, i
     if (WIDE) {
         unsigned long long h, l, *w = bins + kWideWords * e;
         fixed_parts(b.w, h, l);
+        // Where many of a warp's particles go where its first one goes (a few momenta
+        // and cells, as after an injection) one lane adds for them, in 16-bit limbs:
+        // atomics of one address wait for one another (4e6 particles, 50, 90 and
+        // 100 % of them in one bin: 3.0, 4.6 and 5.0 -> 1.9, 0.82 and 0.35 ms; none
+        // in particular, 1e4 bins: 0.19 ms either way).
+        const unsigned here = __activemask();
+        const unsigned e0 = __shfl_sync(here, (unsigned)e, __ffs(here) - 1);
+        const unsigned group = __ballot_sync(here, (unsigned)e == e0);
+        if ((unsigned)e == e0 && __popc(group) >= 4) {
+            const bool leads = (threadIdx.x & 31) == __ffs(group) - 1;
+            if (leads) atomicAdd(w, (unsigned long long)__popc(group));
+#pragma unroll
+            for (int k = 0; k < 8; ++k) {
+                const unsigned limb = (unsigned)((k < 4 ? l >> (16 * k) : h >> (16 * (k - 4))) & 0xffffull);
+                const unsigned sum = __reduce_add_sync(group, limb);
+                if (leads && sum) atomicAdd(w + 1 + k / 2, (unsigned long long)sum << (16 * (k & 1)));
+            }
+            return;
+        }
         atomicAdd(w, 1ull);
         if (l & 0xffffffffull) atomicAdd(w + 1, l & 0xffffffffull);
         if (l >> 32) atomicAdd(w + 2, l >> 32);
