@@ -10,6 +10,9 @@
 #include <new>
 #include <vector>
 
+#include <sys/mman.h>
+#include <unistd.h>
+
 #include "fp64_exact.cuh"
 #include "gpat_internal.h"
 
@@ -1741,6 +1744,25 @@ int gpat_local_distribution_dims(gpat_handle_t *h, const gpat_local_dist_t *spec
     return GPAT_OK;
 }
 
+// Has the pages of a host buffer present, contents as they are.  A copy from the
+// device into a new array has every page faulted in on its way (local distribution
+// of 1e6 bins into two new arrays of 8 MB: 11.6 ms, 0.9 with the pages populated at
+// once before; 3.3e7 bins 36.5 -> 23.7 ms).  A read and a write of each page would
+// fault twice: 2.7 against 0.25 ms for 8 MB.  Nothing depends on it: where the system
+// refuses, the copy does as before.
+static void populate(void *p, size_t bytes) {
+#ifdef MADV_POPULATE_WRITE
+    const uintptr_t page = (uintptr_t)sysconf(_SC_PAGESIZE);
+    if (!p || bytes < 65536) return;
+    const uintptr_t lo = (uintptr_t)p & ~(page - 1);
+    const uintptr_t hi = ((uintptr_t)p + bytes + page - 1) & ~(page - 1);
+    (void)madvise(reinterpret_cast<void *>(lo), hi - lo, MADV_POPULATE_WRITE);
+#else
+    (void)p;
+    (void)bytes;
+#endif
+}
+
 extern "C++" {
 // Runs a binning (wide: launch_local_dist's words, otherwise zeroed (count, whi,
 // wlo) triples) into a device buffer, turns it into weights and counts there,
@@ -1777,6 +1799,8 @@ static int run_bins(gpat_handle_t *h, size_t nbins, bool wide, Launch launch, do
     cudaError_t e = cudaSuccess;
     if (!wide) e = cudaMemsetAsync(bins, 0, sizeof(unsigned long long) * words, h->stream);
     if (e == cudaSuccess) e = launch(bins);
+    populate(f, sizeof(double) * nbins);   // while the GPU works
+    populate(c, sizeof(uint64_t) * nbins);
     for (size_t b = 0; b < nbins && e == cudaSuccess; b += kBinsOut) {
         const size_t m = std::min(kBinsOut, nbins - b);
         e = launch_bins_out(bins + per * b, m, (int)per, df, dc, h->stream);
