@@ -1327,7 +1327,7 @@ int gpat_put_particles(gpat_handle_t *h, const gpat_particles_t *src, int64_t n)
     const bool on_gpu = n > 16384;
     if (on_gpu) {
         CK(cudaMemsetAsync(&h->dcnt->tag_top, 0, 2 * sizeof(unsigned int), h->stream));
-        CK(launch_tag_range(D, n, h->dcnt, h->stream));
+        CK(launch_tag_range(D, n, h->dcnt, h->sm_count, h->stream));
         CK(cudaMemcpyAsync(&h->hcnt.tag_top, &h->dcnt->tag_top, 2 * sizeof(unsigned int),
                            cudaMemcpyDeviceToHost, h->stream));
     }
@@ -1695,7 +1695,8 @@ int gpat_calc_particle_distributions(gpat_handle_t *h, double *fglobal, uint64_t
     if (!h) return GPAT_ERR_ARG;
     CK(cudaSetDevice(h->device));
     const int npp = h->prm.npp_global;
-    CK(launch_histogram(h->P[h->cur], h->n, npp, h->prm.pmin, h->prm.pmax, h->dbins, h->stream));
+    CK(launch_histogram(h->P[h->cur], h->n, npp, h->prm.pmin, h->prm.pmax, h->dbins,
+                        h->sm_count, h->stream));
     std::vector<unsigned long long> b(3 * (size_t)npp);
     CK(cudaMemcpyAsync(b.data(), h->dbins, sizeof(unsigned long long) * b.size(),
                        cudaMemcpyDeviceToHost, h->stream));
@@ -1868,7 +1869,7 @@ int gpat_calc_particle_distributions_mu(gpat_handle_t *h, int32_t nmu, double *f
     const MuDistArgs a = mu_args(h, nmu, 0);
     const size_t nbins = (size_t)nmu * (size_t)a.npp;
     return run_bins(h, nbins, false, [&](unsigned long long *bins) {
-        return launch_mu_dist(h->P[h->cur], h->n, a, bins, nbins, h->stream);
+        return launch_mu_dist(h->P[h->cur], h->n, a, bins, nbins, h->sm_count, h->stream);
     }, fglobal, counts);
 }
 
@@ -1879,7 +1880,7 @@ int gpat_calc_escaped_distributions_mu(gpat_handle_t *h, int32_t nmu, double *fe
     const MuDistArgs a = mu_args(h, nmu, 1);
     const size_t nbins = (size_t)nmu * (size_t)a.npp * 2 * (size_t)h->prm.ndim;
     return run_bins(h, nbins, false, [&](unsigned long long *bins) {
-        return launch_mu_dist(h->E, h->ne, a, bins, nbins, h->stream);
+        return launch_mu_dist(h->E, h->ne, a, bins, nbins, h->sm_count, h->stream);
     }, fescaped, counts);
 }
 
@@ -2070,7 +2071,7 @@ int gpat_quick_check(gpat_handle_t *h, double out[8]) {
     const size_t len = offsetof(DevCounters, status) - off;
     CK(cudaMemcpyAsync(reinterpret_cast<char *>(h->dcnt) + off, reinterpret_cast<char *>(&z) + off,
                        len, cudaMemcpyHostToDevice, h->stream));
-    CK(launch_quick_check(h->P[h->cur], h->n, h->dcnt, h->stream));
+    CK(launch_quick_check(h->P[h->cur], h->n, h->dcnt, h->sm_count, h->stream));
     int rc = pull_counters(h);
     if (rc) return rc;
     const DevCounters &c = h->hcnt;

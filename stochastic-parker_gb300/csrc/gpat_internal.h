@@ -251,7 +251,7 @@ cudaError_t launch_scatter_aux(const float *src, float *aux, int comp, size_t nc
 cudaError_t launch_fill(float *a, float v, size_t n, cudaStream_t s);
 // Raises cnt->tag_top to the largest tag_injected + 1 and cnt->tag_low to the
 // largest -tag_splitted, where these are above 0.
-cudaError_t launch_tag_range(const DevParticles &P, int64_t n, DevCounters *cnt, cudaStream_t s);
+cudaError_t launch_tag_range(const DevParticles &P, int64_t n, DevCounters *cnt, int sm_count, cudaStream_t s);
 cudaError_t launch_mover_fp64(const MoverArgs &a, int sm_count, cudaStream_t s);
 // The same in teams of kMoverTeam lanes, for launch_mover_fp64.
 constexpr int kMoverTeam = 8;
@@ -422,7 +422,7 @@ struct MuDistArgs {
     int npp, nmu, by_face;
 };
 cudaError_t launch_mu_dist(const DevParticles &P, int64_t n, const MuDistArgs &a,
-                           unsigned long long *bins, size_t nbins, cudaStream_t s);
+                           unsigned long long *bins, size_t nbins, int sm_count, cudaStream_t s);
 // Splitting: children appended after n in parent order, at most cap - n.
 // With tracking on, tracked parents follow split_particle's tracking branch.
 cudaError_t launch_split_particles(const DevParticles &P, int64_t n, int64_t cap,
@@ -475,10 +475,10 @@ cudaError_t launch_cell_sort(const DevParticles &src, const DevParticles &dst, i
                              const EscHist &esc, cudaStream_t s);
 // Global f(p) histogram into (count, whi, wlo) triples per bin (zeroed here).
 cudaError_t launch_histogram(const DevParticles &P, int64_t n, int npp, double pmin,
-                             double pmax, unsigned long long *bins, cudaStream_t s);
+                             double pmax, unsigned long long *bins, int sm_count, cudaStream_t s);
 // quick_check reductions into cnt (wsum, dtsum, dt_min, dt_max).
 cudaError_t launch_quick_check(const DevParticles &P, int64_t n, DevCounters *cnt,
-                               cudaStream_t s);
+                               int sm_count, cudaStream_t s);
 
 // Learned splitting launchers (learned.cu).
 size_t mlp_shared_bytes();

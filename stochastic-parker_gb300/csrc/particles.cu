@@ -1129,7 +1129,7 @@ cudaError_t launch_sync_tracked(const TrackArgs &trk, cudaStream_t s) {
 }
 
 cudaError_t launch_histogram(const DevParticles &P, int64_t n, int npp, double pmin, double pmax,
-                             unsigned long long *bins, cudaStream_t s) {
+                             unsigned long long *bins, int sm_count, cudaStream_t s) {
     MuDistArgs a{};
     a.pmin = pmin;
     a.pmax = pmax;
@@ -1138,7 +1138,7 @@ cudaError_t launch_histogram(const DevParticles &P, int64_t n, int npp, double p
     a.dmu = 1.0;
     a.npp = npp;
     a.nmu = 0;   // one bin for all pitch angles
-    return launch_mu_dist(P, n, a, bins, (size_t)npp, s);
+    return launch_mu_dist(P, n, a, bins, (size_t)npp, sm_count, s);
 }
 
 // The bins of particle i for one local-distribution parameter set
@@ -1371,7 +1371,7 @@ cudaError_t launch_local_escaped(const DevParticles &P, int64_t n, const LocalDi
 }
 
 cudaError_t launch_mu_dist(const DevParticles &P, int64_t n, const MuDistArgs &a,
-                           unsigned long long *bins, size_t nbins, cudaStream_t s) {
+                           unsigned long long *bins, size_t nbins, int sm_count, cudaStream_t s) {
     cudaError_t e = cudaMemsetAsync(bins, 0, sizeof(unsigned long long) * 3 * nbins, s);
     if (e != cudaSuccess || n <= 0) return e;
     const MuBins g{a, make_log_bins(a.pmin_log, a.dp_log), make_even_bins(-1.0, a.dmu)};
@@ -1384,7 +1384,8 @@ cudaError_t launch_mu_dist(const DevParticles &P, int64_t n, const MuDistArgs &a
         // Every block adds its table to the global one: four blocks per SM as
         // far as they fit, fewer where a table costs more than its particles.
         int64_t blocks = (n + 255) / 256;
-        const int64_t most = std::max<int64_t>(152, std::min<int64_t>(608, n / (4 * (int64_t)nbins)));
+        const int64_t most = std::max<int64_t>(
+            sm_count, std::min<int64_t>(4 * sm_count, n / (4 * (int64_t)nbins)));
         if (blocks > most) blocks = most;
         bins_shared_kernel<<<(unsigned)blocks, 256, shmem, s>>>(P, n, g, (int)nbins, bins);
     } else {
@@ -1393,10 +1394,11 @@ cudaError_t launch_mu_dist(const DevParticles &P, int64_t n, const MuDistArgs &a
     return cudaGetLastError();
 }
 
-cudaError_t launch_quick_check(const DevParticles &P, int64_t n, DevCounters *cnt, cudaStream_t s) {
+cudaError_t launch_quick_check(const DevParticles &P, int64_t n, DevCounters *cnt, int sm_count,
+                               cudaStream_t s) {
     if (n <= 0) return cudaSuccess;
     int64_t blocks = (n + 255) / 256;
-    if (blocks > 608) blocks = 608;
+    if (blocks > 4 * sm_count) blocks = 4 * sm_count;
     quick_check_kernel<<<(unsigned)blocks, 256, 0, s>>>(P, n, cnt);
     return cudaGetLastError();
 }
@@ -1421,9 +1423,10 @@ __global__ void __launch_bounds__(256) tag_range_kernel(const DevParticles P, in
 
 }  // namespace
 
-cudaError_t launch_tag_range(const DevParticles &P, int64_t n, DevCounters *cnt, cudaStream_t s) {
+cudaError_t launch_tag_range(const DevParticles &P, int64_t n, DevCounters *cnt, int sm_count,
+                             cudaStream_t s) {
     if (n <= 0) return cudaSuccess;
-    const unsigned g = (unsigned)std::min<int64_t>((n + 255) / 256, 608);
+    const unsigned g = (unsigned)std::min<int64_t>((n + 255) / 256, 4 * sm_count);
     tag_range_kernel<<<g, 256, 0, s>>>(P, n, cnt);
     return cudaGetLastError();
 }
