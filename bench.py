@@ -498,8 +498,10 @@ def run_ours(args, world, rank, local):
                              f"particle state {state_mb:.0f} MB)",
                        "parallelism": f"replicas x{world}"},
             "clocks": clk,
-            # per step: mover launches, a 5-kernel binning after each, split (3), f(p) (1)
-            "gpu_launches": int(round(sum(6 * l + 4 for l in kernel_launches))) if prec
+            # per step: mover launches, a binning of 5 kernels (6 from 600 000 particles
+            # on) after each, split (3), f(p) (1)
+            "gpu_launches": int(round(sum((7 if w.nptl >= 600_000 else 6) * l + 4
+                                          for l in kernel_launches))) if prec
             else 8 * args.steps,
             "e2e": {"value": e2e_value, "unit": UNIT,
                     "h2d_bytes_per_step": e2e_h2d // max(1, args.e2e_steps),
@@ -951,6 +953,75 @@ def other_configs(args, local) -> dict:
     return out
 
 
+# What the line on standard output may take; readers that keep the end of a log then
+# have all of it.
+LINE_BYTES = 3000
+CONTRACT_KEYS = ("metric", "value", "unit", "n_gpus", "steps", "warmup", "ms_per_step",
+                 "higher_is_better", "scaling", "vs_baseline", "dtype", "data", "impl", "config",
+                 "clocks", "gpu_launches", "e2e")
+
+
+def rounded(x):
+    """Figures to six digits, long texts and lists cut."""
+    if isinstance(x, float):
+        return float(f"{x:.6g}")
+    if isinstance(x, dict):
+        return {k: rounded(v) for k, v in x.items()}
+    if isinstance(x, (list, tuple)):
+        return [rounded(v) for v in x[:8]]
+    return x[:100] if isinstance(x, str) else x
+
+
+def summary(line) -> dict:
+    """The figures of a workload's own line that its summary keeps."""
+    out = {k: line[k] for k in ("error", "value", "unit", "ms_per_step") if k in line}
+    roof = line.get("roofline") or {}
+    out.update({k: roof[k] for k in ("bound", "frac") if k in roof})
+    errs = [abs(r["tail_err"]) for r in line.get("per_run_fp_error") or []
+            if isinstance(r.get("tail_err"), (int, float))]
+    if errs:
+        out["runs_compared"], out["max_abs_tail_err"] = len(errs), max(errs)
+    learned = line.get("learned_splitting") or {}
+    out.update({k: learned[k] for k in ("ess_per_s_learned_over_fixed",
+                                        "ess_per_s_learned_over_plain") if k in learned})
+    return out
+
+
+def short_line(line) -> dict:
+    """The line of standard output: the contract's keys whole, of the rest the figures,
+    and of the other configurations their summaries."""
+    out = {k: line[k] for k in CONTRACT_KEYS if k in line}
+    rest = {k: v for k, v in line.items() if k not in out}
+    roof = rest.pop("roofline", None)
+    if roof:
+        hbm = roof.get("hbm") or {}
+        out["roofline"] = rounded({**{k: roof[k] for k in ("bound", "achieved", "peak", "unit", "frac",
+                                                           "traffic", "kernel_steps_per_s", "kernel")
+                                      if k in roof}, "hbm_frac": hbm.get("frac")})
+    acc = rest.pop("accuracy", None)
+    if acc:
+        out["accuracy"] = rounded({k: v for k, v in acc.items() if not isinstance(v, (list, str))})
+    for key in ("cpu_baseline", "fp64_gpu"):
+        if rest.get(key):
+            out[key] = rounded(rest.pop(key))
+    out.update(rounded({k: v for k, v in summary(rest).items() if k not in out}))
+    configs = rest.pop("configs", None)
+    if configs:
+        out["configs"] = {k: rounded(summary(v)) for k, v in configs.items()}
+    for key in ("configs", "fp64_gpu", "cpu_baseline", "accuracy", "roofline"):
+        if len(json.dumps(out)) <= LINE_BYTES:
+            break
+        out.pop(key, None)
+    return out
+
+
+def emit(line):
+    """The whole line, with every figure, on standard error; the short one on standard
+    output."""
+    print("bench: details " + json.dumps(line), file=sys.stderr, flush=True)
+    print(json.dumps(short_line(line)), flush=True)
+
+
 def main():
     args = parse_args()
     world, rank, local = dist_setup()
@@ -959,18 +1030,18 @@ def main():
     elif args.workload == "batched_shock_2d":
         line = run_batch(args, world, rank, local)
         if line is not None:
-            print(json.dumps(line), flush=True)
+            emit(line)
     elif args.workload == "learned_3d":
         line = run_learned(args, world, rank, local)
         if line is not None:
-            print(json.dumps(line), flush=True)
+            emit(line)
     else:
         line = run_ours(args, world, rank, local)
         if line is not None and args.workload == "turbulent_shock_2d" and not args.no_extras \
                 and world == 1:
             line["configs"] = other_configs(args, local)
         if line is not None:
-            print(json.dumps(line), flush=True)
+            emit(line)
     if world > 1:
         import torch.distributed as dist
         dist.destroy_process_group()
