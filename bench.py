@@ -247,30 +247,31 @@ def measured_peaks() -> dict:
     return {"hbm_gbs": 6800.0, "source": "fallback"}
 
 
-# From the ncu captures summarised in profiles/ (commands there): DRAM bytes
-# (read + write) per push of the mover kernel at the bench's particle
-# density (3D: two late launches of 3e7 particles), and the L1TEX throughput (percent of peak, active cycles) of the
-# full capture, which ncu names as the binding unit of the gather movers.
+# Of one whole interval of a workload at its full particle count, per counted push
+# (profiles/mover_traffic.md, with the commands): DRAM bytes read and written, and
+# wavefronts of up to 128 bytes of the L1TEX data pipe, of which an SM does one per
+# clock and which bounds the gather movers.  Both depend on how many particles share
+# a cell, so the DRAM figure is given out for that workload and count alone.
 NCU_MOVER = {
-    ("global", 2): {"dram_bytes_per_push": 0.947, "l1tex_pct": 71.5,
-                    "profile": "profiles/case_times.md"},
-    ("global", 3): {"dram_bytes_per_push": 44.0, "l1tex_pct": 71.6,
-                    "profile": "profiles/case_times.md"},
+    2: {"workload": "turbulent_shock_2d_2048x2048", "particles": 10_000_000,
+        "dram_bytes_per_push": 0.933, "wavefronts_per_push": 4.18,
+        "profile": "profiles/mover_traffic.md"},
+    3: {"workload": "turbulence_3d_256^3", "particles": 100_000_000,
+        "dram_bytes_per_push": 14.0, "wavefronts_per_push": 15.3,
+        "profile": "profiles/mover_traffic.md"},
 }
-# The L1TEX data path per push and per clock, in data-pipe wavefronts of up to
-# 128 bytes, one per clock per SM.  Global-gather movers: groups of lanes read
-# a record's sectors of one line together, and the captures count 4.35
-# wavefronts per push in 2D (1.114e9 for 2.56e8 pushes) and about 14 in 3D
-# (1.189e9 for 8.5e7, the exchange through shared memory included).  Brick
-# movers read 16-byte chunks from shared memory (nominal; bank conflicts cost
-# more).
-L1_MODEL = {("global", 2): {"bytes_per_push": 4.35 * 128, "bytes_per_clk_sm": 128},
-            ("global", 3): {"bytes_per_push": 14 * 128, "bytes_per_clk_sm": 128},
+# Bytes per push on that pipe.  Global-gather movers: the wavefronts above; brick
+# movers read 16-byte chunks from shared memory (nominal; bank conflicts cost more).
+L1_MODEL = {("global", 2): {"bytes_per_push": NCU_MOVER[2]["wavefronts_per_push"] * 128,
+                            "bytes_per_clk_sm": 128},
+            ("global", 3): {"bytes_per_push": NCU_MOVER[3]["wavefronts_per_push"] * 128,
+                            "bytes_per_clk_sm": 128},
             ("tile", 2): {"bytes_per_push": 4 * 64, "bytes_per_clk_sm": 128},
             ("tile", 3): {"bytes_per_push": 8 * (5 * 16 + 4), "bytes_per_clk_sm": 128}}
 
 
-def roofline_of(kind, ndim, avg_ms, avg_steps, avg_n, sm_count, sm_mhz, peaks) -> dict:
+def roofline_of(kind, ndim, avg_ms, avg_steps, avg_n, sm_count, sm_mhz, peaks, workload=None,
+                particles=None) -> dict:
     """Roofline of one mover launch: the L1TEX data path is the bound (ncu),
     HBM is reported beside it on the algorithmic bytes."""
     secs = avg_ms / 1e3
@@ -278,17 +279,18 @@ def roofline_of(kind, ndim, avg_ms, avg_steps, avg_n, sm_count, sm_mhz, peaks) -
     l1_bytes = avg_steps * m["bytes_per_push"]
     l1_peak = sm_count * m["bytes_per_clk_sm"] * (sm_mhz or 2070.0) * 1e6 / 1e9
     alg = avg_steps * GATHER_BYTES_PER_STEP[ndim] + avg_n * STATE_BYTES_PER_PARTICLE
-    ncu = NCU_MOVER.get((kind, ndim), {})
-    dram = ncu.get("dram_bytes_per_push")
+    ncu = NCU_MOVER[ndim] if kind == "global" else {}
+    same = ncu and (workload, particles) == (ncu["workload"], ncu["particles"])
+    dram = ncu["dram_bytes_per_push"] if same else None
     what = "L1TEX data pipe" if kind == "global" else "nominal shared-memory rate"
     peak_source = (f"{what}: one wavefront of 128 bytes per clock per SM x {sm_count} SMs x "
                    f"median sampled SM clock {sm_mhz} MHz")
     return {"bound": "l1", "achieved": l1_bytes / secs / 1e9, "peak": l1_peak, "unit": "GB/s",
             "frac": l1_bytes / secs / 1e9 / l1_peak, "peak_source": peak_source,
             "traffic": dram * avg_steps if dram is not None else None,
-            "traffic_source": ncu.get("profile"),
-            "ncu_l1tex_throughput_pct": ncu.get("l1tex_pct"),
+            "traffic_source": ncu["profile"] if same else None,
             "l1_bytes_per_push": m["bytes_per_push"],
+            "l1_measured_at": f"{ncu['workload']}, {ncu['particles']} particles" if ncu else "nominal",
             "kernel_ms_per_launch": avg_ms, "steps_per_launch": avg_steps,
             "kernel_steps_per_s": avg_steps / secs,
             "hbm": {"achieved": alg / secs / 1e9, "peak": peaks["hbm_gbs"],
@@ -296,8 +298,8 @@ def roofline_of(kind, ndim, avg_ms, avg_steps, avg_n, sm_count, sm_mhz, peaks) -
                     "algorithmic_bytes_per_push": GATHER_BYTES_PER_STEP[ndim],
                     "state_bytes_per_particle": STATE_BYTES_PER_PARTICLE},
             "note": "achieved = L1 data-pipe wavefronts (128 B) per push x pushes / launch "
-                    "time, against one per clock and SM; ncu_l1tex_throughput_pct is the "
-                    "unit's measured busy share; hbm = algorithmic bytes (corners x stored field "
+                    "time, against one per clock and SM, counted where l1_measured_at says; "
+                    "hbm = algorithmic bytes (corners x stored field "
                     "arrays x 4 B + FP64 state) over measured HBM"}
 
 
@@ -475,7 +477,7 @@ def run_ours(args, world, rank, local):
     kind = "tile" if tiles else "global"
     sm_count = torch.cuda.get_device_properties(dev).multi_processor_count
     roofline = roofline_of(kind, ndim, avg_ms, avg_steps, avg_n, sm_count, clk.get("sm_mhz"),
-                           peaks)
+                           peaks, w.name if prec else None, w.nptl)
     roofline["kernel"] = (f"mover_tile_kernel<{ndim}> + mover_overflow_kernel<{ndim}>" if tiles
                           else f"mover_{args.precision}_kernel<{ndim}>")
     roofline["mover_launches_per_interval"] = launches

@@ -89,3 +89,21 @@ def test_other_workloads_lines(bench):
     assert short["runs_compared"] == 64 and short["value"] == batch["value"]
     failed = bench.short_line(dict(metric="m", value=None, configs={"a": {"error": "out of memory"}}))
     assert failed["configs"] == {"a": {"error": "out of memory"}}
+
+
+def test_traffic_only_where_it_was_counted(bench):
+    """DRAM bytes per push depend on the particles per cell: given for the workload and
+    the count of the capture, not for others, not for the brick mover."""
+    peaks = {"hbm_gbs": 6800.0, "source": "fallback"}
+    for ndim, ncu in bench.NCU_MOVER.items():
+        args = ("global", ndim, 25.0, 1.25e9, 1e7, 152, 2070.0, peaks)
+        own = bench.roofline_of(*args, ncu["workload"], ncu["particles"])
+        assert own["traffic"] == ncu["dram_bytes_per_push"] * 1.25e9
+        assert own["traffic_source"] == ncu["profile"] and (REPO / ncu["profile"]).exists()
+        assert own["achieved"] == pytest.approx(ncu["wavefronts_per_push"] * 128 * 1.25e9 / 25e-3 / 1e9)
+        for other in ((ncu["workload"], ncu["particles"] // 10), ("other", ncu["particles"]), ()):
+            assert bench.roofline_of(*args, *other)["traffic"] is None
+        assert str(ncu["particles"]) in own["l1_measured_at"]
+    tile = bench.roofline_of("tile", 3, 25.0, 1.25e9, 1e7, 152, 2070.0, peaks, "turbulence_3d_256^3",
+                             100_000_000)
+    assert tile["traffic"] is None and tile["l1_measured_at"] == "nominal"
