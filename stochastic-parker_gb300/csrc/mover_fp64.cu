@@ -1580,9 +1580,13 @@ __device__ __forceinline__ void track_push(const MoverArgs &a, const State &s, i
 // different numbers of pushes (adaptive steps, start times spread over the
 // interval), so the grid is persistent and the loop turns once per push: a
 // lane whose particle has finished takes the next one from a counter (the
-// longest first, order_particles) and the warp's instructions stay full.  The landing's redone push runs through the
-// same code as an ordinary one.  What a particle computes does not depend on
+// longest first, order_bin) and the warp's instructions stay full.  The landing's
+// redone push runs through the same code as an ordinary one.  What a particle computes does not depend on
 // its lane.
+// Taking one costs the warp a wait for memory, so lanes whose particles had fewer
+// pushes than kRefillAfter wait for the warp's others.
+constexpr uint32_t kRefillAfter = 3;
+
 template <int NDIM, bool FT, bool FULL, bool GRID, bool I3>
 __global__ void __launch_bounds__(128) mover_fp64_kernel(const MoverArgs a) {
     Acc acc = {0, 0, 0, 0, 0};
@@ -1602,6 +1606,9 @@ __global__ void __launch_bounds__(128) mover_fp64_kernel(const MoverArgs a) {
         while (more) {
             const unsigned need = __ballot_sync(0xffffffffu, !have && taker);
             if (need == 0u) break;
+            if (__any_sync(0xffffffffu, have) &&
+                !__any_sync(0xffffffffu, !have && taker && pushes >= kRefillAfter))
+                break;
             const int leader = __ffs(need) - 1;
             unsigned long long base = 0;
             if (lane == leader) base = atomicAdd(&a.cnt->next, (unsigned long long)__popc(need));
