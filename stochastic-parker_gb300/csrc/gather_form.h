@@ -25,6 +25,11 @@ inline double gather_step(int ndim, double kpara0, double dt_max, double dx, dou
     return std::fmin(std::sqrt(2.0 * std::fabs(kpara0) * dt_max) / h, 0.5);
 }
 
+// Whether particles end their pushes near a face of the box often (MixedConsts::
+// all_bounds): 2D 64^2, skipping the test over not, steps of 0.1 and less 0.94, 0.3
+// 1.1 to 1.3.
+inline int long_steps(double step, bool kappa_rises) { return step >= (kappa_rises ? 0.05 : 0.2); }
+
 // Gathering by groups of lanes spares the L1 data pipe, and costs shuffles and
 // weights computed twice (2D) or a turn through shared memory (3D).  It gains
 // where that pipe is the bound: two frames, records that neighbouring lanes do not
@@ -55,7 +60,8 @@ inline bool gathers_in_groups(const GatherLoad &g) {
         return per_cell < 1.0 && g.cells >= 4e5;
     }
     // a launch that leaves a particle a whole group of lanes (spread_of)
-    if (2 * g.n <= (int64_t)g.sm_count * 128 * 4 || per_cell < 0.3) return true;
+    if (2 * g.n <= (int64_t)g.sm_count * 128 * 4) return true;
+    if (per_cell < 0.3) return true;
     if (g.two_frames) return g.step >= (per_cell < 4.0 ? 0.06 : 0.015);
     return g.step >= (per_cell < 4.0 ? 0.12 : 0.06);
 }

@@ -2245,6 +2245,9 @@ int batch_prepare(gpat_batch_t *b, const int *tframes, int nlgc, double kperp_kp
         BatchRun &d = b->desc[r];
         d.a = mixed_run_args(a);
         d.k = make_mixed_consts(a);
+        // in the persistent kernel lanes that go apart meet late: 4 runs of 30 000
+        // particles, 64^2 cells, steps of 0.1 cells 22.4 -> 18.1 ms
+        d.k.all_bounds = 1;
         d.P[0] = h->P[0];
         d.P[1] = h->P[1];
         b->host_ull[r] = (unsigned long long)h->n;

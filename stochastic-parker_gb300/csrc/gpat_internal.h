@@ -153,6 +153,7 @@ struct MixedConsts {
     float pfloor;                      // 0.25 p0
     float acc[6];                      // acceleration region, box fractions
     float acc_off[3], acc_scale[3];    // cell -> box fraction: (c + off) * scale
+    int all_bounds;                    // move_particle: every lane through the boundary test
 };
 
 // What the split-precision mover reads besides MixedConsts and the particle

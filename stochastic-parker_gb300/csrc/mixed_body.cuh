@@ -71,15 +71,21 @@ __device__ __forceinline__ void boundary(const MixedRunArgs &a, const MixedConst
     if (NDIM == 3) bc_axis(q.cz, q.fz, k.nz, ext, a.pbcz, -5, -6, flag, a, w);
 }
 
+// all: the lanes go through the boundary test together; else those whose particle is
+// in one of the box's own cells, where it finds nothing, skip it.  In move_warp the
+// lanes meet at the gather right after it.  In move_particle those that went through
+// it stay apart for the push, so it is skipped for short steps only, where few do
+// (MixedConsts::all_bounds; brick mover, 3D 64^3, steps of 0.01 and 0.1 cells 5.8 -> 4.9
+// and 6.7 -> 5.9 ms, of half a cell 37.6 -> 41.4; a barrier there would have lanes land
+// apart: 1e6 particles of 10 pushes 0.51 -> 0.66 ms).
 template <int NDIM>
 __device__ __forceinline__ void negp_or_boundary(const MixedRunArgs &a, const MixedConsts &k, Pos &q,
-                                                 float p, int &flag, const double *w) {
+                                                 float p, bool all, int &flag, const double *w) {
     if (p < 0.0f) {
         flag = 0;
         atomic_add_fixed(&a.cnt->negp_hi, &a.cnt->negp_lo, *w);
-    } else if ((unsigned)q.cx >= (unsigned)k.nx || (unsigned)q.cy >= (unsigned)k.ny ||
+    } else if (all || (unsigned)q.cx >= (unsigned)k.nx || (unsigned)q.cy >= (unsigned)k.ny ||
                (NDIM == 3 && (unsigned)q.cz >= (unsigned)k.nz)) {
-        // not in one of the box's own cells
         boundary<NDIM>(a, k, q, true, flag, w);
     }
 }
@@ -635,13 +641,7 @@ __device__ __forceinline__ uint32_t move_particle(const MixedRunArgs &a, const M
         while (alive && target_d < a.limit) {
             const float target = (float)target_d;
             while (tau - tc < target && flag == 1) {
-                // Lanes whose particle is outside the box's cells would stay apart
-                // for the push: they meet the others again.  Brick mover, steps of
-                // half a cell, 3D 64^3: 41.4 -> 35.7 ms (37.6 with every lane through
-                // the boundary test); 2D 64^2: 58.6 -> 54.9 (56.6).
-                const unsigned here = __activemask();
-                negp_or_boundary<NDIM>(a, k, q, p - pc, flag, wp);
-                __syncwarp(here);
+                negp_or_boundary<NDIM>(a, k, q, p - pc, k.all_bounds != 0, flag, wp);
                 if (flag != 1) break;
                 if (limit != 0 && pushes >= limit) {
                     paused = true;   // between pushes: the next launch resumes from t
@@ -719,7 +719,7 @@ __device__ __forceinline__ uint32_t move_particle(const MixedRunArgs &a, const M
                     nsp = (nsp + 1) % a.nsteps_interval;
                 }
                 dt = dt_old;
-                negp_or_boundary<NDIM>(a, k, q, p - pc, flag, wp);
+                negp_or_boundary<NDIM>(a, k, q, p - pc, k.all_bounds != 0, flag, wp);
             } else if (flag == 1 && tau - tc == target) {
                 landed_at = target_d;   // reached the target without overshoot
             }
@@ -820,7 +820,7 @@ __device__ __forceinline__ uint32_t move_warp(const MixedRunArgs &a, const Mixed
         bool want = false, fixed = false;
         while (alive && flag == 1) {
             if (tau - tc < target) {
-                negp_or_boundary<NDIM>(a, k, q, p - pc, flag, P.weight + i);
+                negp_or_boundary<NDIM>(a, k, q, p - pc, false, flag, P.weight + i);
                 if (flag != 1) break;
                 if (limit != 0 && pushes >= limit) {
                     paused = true;   // between pushes: the next launch resumes from t
@@ -847,7 +847,7 @@ __device__ __forceinline__ uint32_t move_warp(const MixedRunArgs &a, const Mixed
                     fixed = true;
                     break;
                 }
-                negp_or_boundary<NDIM>(a, k, q, p - pc, flag, P.weight + i);
+                negp_or_boundary<NDIM>(a, k, q, p - pc, false, flag, P.weight + i);
             } else if (tau - tc == target) {
                 landed = true;         // reached the target without overshoot
                 landed_d = target_d;
@@ -890,7 +890,7 @@ __device__ __forceinline__ uint32_t move_warp(const MixedRunArgs &a, const Mixed
                 tau = target; tc = 0.0f;
                 landed = true;
                 landed_d = target_d;
-                negp_or_boundary<NDIM>(a, k, q, p - pc, flag, P.weight + i);
+                negp_or_boundary<NDIM>(a, k, q, p - pc, false, flag, P.weight + i);
                 target_d = target_d + a.dt_fine;
                 target = (float)target_d;
                 alive = target_d < a.limit;

@@ -52,6 +52,8 @@ MixedConsts make_mixed_consts(const MoverArgs &a) {
     k.acc_scale[0] = (float)(a.dx / a.cfg_lx);
     k.acc_scale[1] = (float)(a.dy / a.cfg_ly);
     k.acc_scale[2] = (float)(a.dz / a.cfg_lz);
+    k.all_bounds = long_steps(gather_step(a.ndim, a.kpara0, a.dt_max, a.dx, a.dy, a.dz),
+                              a.momentum_dependency != 0);
     return k;
 }
 

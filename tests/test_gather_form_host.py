@@ -46,6 +46,8 @@ int main() {
     std::printf("%.3f %.3f %.3f\n", gather_step(2, 1.0, 1.0, d, d, 1.0),
                 gather_step(3, 0.0, 1.0, d, d, d), gather_step(3, d * d / 8, 0.01, d, 2 * d, d / 2));
     std::printf("%d\n", (int)gathers_in_groups({3, false, 1, 8.0, 0.125, nan, 152}));
+    std::printf("%d %d %d %d\n", long_steps(0.1, false), long_steps(0.3, false), long_steps(0.1, true),
+                long_steps(0.01, true));
     return 0;
 }
 """
@@ -67,3 +69,4 @@ def test_forms_at_the_measured_points(tmp_path):
     # 0.1 = sqrt(2 (d^2 / 8) 0.01) / (d / 2)
     assert out[len(POINTS)] == "0.500 0.000 0.100"
     assert out[len(POINTS) + 1] in ("0", "1")
+    assert out[len(POINTS) + 2] == "0 1 1 0"
