@@ -15,6 +15,7 @@ struct GatherLoad {
     double per_cell;   // particles of the run per cell
     double step;       // what diffusion along B moves a particle in a longest step, in cells
     int sm_count;
+    double pushes;     // of a particle in the launch, at most
 };
 
 // Half a cell is what the step's diffusion limit allows.  At p0: with kappa rising
@@ -53,14 +54,16 @@ inline int long_steps(double step, bool kappa_rises) { return step >= (kappa_ris
 //     and 32: 1.06 to 1.11; 0.1: 1.0 to 1.35; 0.3: 1.05 to 1.3; 0.1 a cell 1.04 to 1.4.
 inline bool gathers_in_groups(const GatherLoad &g) {
     const double per_cell = g.per_cell;
+    const bool few = g.pushes <= 16.0;
     if (g.ndim == 2) {
-        if (2 * g.n <= (int64_t)g.sm_count * 128) return false;
+        if (few || 2 * g.n <= (int64_t)g.sm_count * 128) return false;
         if (g.two_frames) return per_cell < 1.0 || g.step >= 0.25;
         if (g.step >= 0.45) return g.cells >= 4e5 || g.n >= 40000;
         return per_cell < 1.0 && g.cells >= 4e5;
     }
     // a launch that leaves a particle a whole group of lanes (spread_of)
     if (2 * g.n <= (int64_t)g.sm_count * 128 * 4) return true;
+    if (few) return false;
     if (per_cell < 0.3) return true;
     if (g.two_frames) return g.step >= (per_cell < 4.0 ? 0.06 : 0.015);
     return g.step >= (per_cell < 4.0 ? 0.12 : 0.06);

@@ -10,7 +10,8 @@ import pytest
 
 CSRC = Path(__file__).resolve().parent.parent / "stochastic-parker_gb300" / "csrc"
 
-# ndim, two frames, grid (nodes a side), particles a cell, step, groups expected
+# ndim, two frames, grid (nodes a side), particles a cell, step, groups expected; the
+# launch makes 128 pushes
 POINTS = [
     (2, 0, 64, 8.0, 0.03, 0), (2, 0, 64, 2.0, 0.3, 0), (2, 0, 256, 2.0, 0.01, 0),
     (2, 0, 256, 0.5, 0.3, 0), (2, 0, 256, 0.1, 0.5, 0), (2, 0, 512, 0.1, 0.5, 0), (2, 0, 64, 2.0, 0.5, 0),
@@ -39,13 +40,18 @@ int main() {
     while (std::scanf("%d %d %lf %lf %lf", &ndim, &two, &side, &ppc, &step) == 5) {
         const double cells = std::pow(side + 4, ndim);
         const int64_t n = (int64_t)(ppc * std::pow(side, ndim));
-        std::printf("%d\n", (int)gathers_in_groups({ndim, two != 0, n, cells, n / cells, step, 152}));
+        std::printf("%d\n", (int)gathers_in_groups({ndim, two != 0, n, cells, n / cells, step, 152, 128.0}));
     }
     const double nan = std::numeric_limits<double>::quiet_NaN(), d = 1.0 / 128;
     // kappa ratio 1: half a cell at most; no diffusion: no step; the smallest side
     std::printf("%.3f %.3f %.3f\n", gather_step(2, 1.0, 1.0, d, d, 1.0),
                 gather_step(3, 0.0, 1.0, d, d, d), gather_step(3, d * d / 8, 0.01, d, 2 * d, d / 2));
-    std::printf("%d\n", (int)gathers_in_groups({3, false, 1, 8.0, 0.125, nan, 152}));
+    std::printf("%d\n", (int)gathers_in_groups({3, false, 1, 8.0, 0.125, nan, 152, nan}));
+    // launches of few pushes, right after a binning: by single lanes, unless each
+    // particle has a group of its own
+    std::printf("%d %d %d\n", (int)gathers_in_groups({2, true, 2000000, 4e6, 0.5, 0.5, 152, 16.0}),
+                (int)gathers_in_groups({3, true, 1000000, 2e6, 0.5, 0.5, 152, 10.0}),
+                (int)gathers_in_groups({3, true, 30000, 2e6, 0.015, 0.5, 152, 10.0}));
     std::printf("%d %d %d %d\n", long_steps(0.1, false), long_steps(0.3, false), long_steps(0.1, true),
                 long_steps(0.01, true));
     return 0;
@@ -69,4 +75,5 @@ def test_forms_at_the_measured_points(tmp_path):
     # 0.1 = sqrt(2 (d^2 / 8) 0.01) / (d / 2)
     assert out[len(POINTS)] == "0.500 0.000 0.100"
     assert out[len(POINTS) + 1] in ("0", "1")
-    assert out[len(POINTS) + 2] == "0 1 1 0"
+    assert out[len(POINTS) + 2] == "0 0 1"
+    assert out[len(POINTS) + 3] == "0 1 1 0"

@@ -16,11 +16,11 @@ KEYS = ("x", "y", "z", "p", "t", "dt", "count_flag", "nsteps_pushed", "rng_ctr",
 BOX = (0.0, 0.0, 0.0, 1.0, 1.0, 1.0)
 
 
-def _engine(ndim, two, step, n, nmax, seed=5, nlgc=False):
+def _engine(ndim, two, step, n, nmax, seed=5, pushes=64):
     cfg = make_mhd_config(n, n, n if ndim == 3 else 1, 0.0, 1.0, 0.0, 1.0, dt_out=0.02, ndim=ndim)
-    dt_max = 0.02 / 64
+    dt_max = 0.02 / pushes
     prm = make_params(ndim=ndim, p0=0.1, pmin=0.1, pmax=1.0, kpara0=(step / n) ** 2 / (2 * dt_max),
-                      kret=0.1, dt_min_rel=1 / 640, dt_max_rel=1 / 64, pbcx=1, pbcy=0, pbcz=0,
+                      kret=0.1, dt_min_rel=0.1 / pushes, dt_max_rel=1 / pushes, pbcx=1, pbcy=0, pbcz=0,
                       momentum_dependency=0, nptl_max=nmax, seed=seed, precision=1,
                       time_interp=int(two), bin_interval=16)
     eng = Engine(prm, cfg, 0)
@@ -68,6 +68,21 @@ def test_the_same_bits_on_both_sides(ndim, two, step, n, total, parts, nlgc):
         idx = np.sort(np.random.default_rng(m).permutation(total)[:m])
         got = _moved(eng, start, idx, **kw)
         at = np.isin(whole["tag_injected"], start["tag_injected"][idx])
+        for k in KEYS:
+            assert np.array_equal(got[k], whole[k][at]), (m, k)
+    eng.close()
+
+
+@pytest.mark.parametrize("ndim,two", [(2, False), (2, True), (3, True)])
+def test_launches_of_few_pushes(ndim, two):
+    """By single lanes as a whole, the last particles of a 3D set by groups."""
+    eng = _engine(ndim, two, 0.5, 20 if ndim == 3 else 128, 60000, pushes=1.2)
+    eng.inject_particles_spatial_uniform(60000, 1e-6, 2, 1.0, 1, BOX, 1.0)
+    start = eng.get_particles()
+    whole = _moved(eng, start, np.arange(60000))
+    for m in (45000, 20000, 300):
+        got = _moved(eng, start, np.arange(m))
+        at = np.isin(whole["tag_injected"], start["tag_injected"][:m])
         for k in KEYS:
             assert np.array_equal(got[k], whole[k][at]), (m, k)
     eng.close()
