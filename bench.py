@@ -984,8 +984,9 @@ def summary(line) -> dict:
     if errs:
         out["runs_compared"], out["max_abs_tail_err"] = len(errs), max(errs)
     learned = line.get("learned_splitting") or {}
-    out.update({k: learned[k] for k in ("ess_per_s_learned_over_fixed",
-                                        "ess_per_s_learned_over_plain") if k in learned})
+    for k in ("ess_per_s_learned_over_fixed", "ess_per_s_learned_over_plain"):
+        if k in learned:   # no particle of the other arm up there: no ratio
+            out[k] = {name: v if v < 1e12 else None for name, v in learned[k].items()}
     return out
 
 

@@ -18,18 +18,20 @@ struct GatherLoad {
     double pushes;     // of a particle in the launch, at most
 };
 
-// Half a cell is what the step's diffusion limit allows.  At p0: with kappa rising
-// with p the others move further, which speaks for groups.
-inline double gather_step(int ndim, double kpara0, double dt_max, double dx, double dy, double dz) {
+// Half a cell is what the step's diffusion limit allows.  Where kappa rises with p,
+// as p^(4/3) or so, twice what it is at p0: particles of sqrt(10) p0.
+inline double gather_step(int ndim, double kpara0, bool kappa_rises, double dt_max, double dx,
+                          double dy, double dz) {
     double h = std::fmin(dx, dy);
     if (ndim == 3) h = std::fmin(h, dz);
-    return std::fmin(std::sqrt(2.0 * std::fabs(kpara0) * dt_max) / h, 0.5);
+    const double step = std::sqrt(2.0 * std::fabs(kpara0) * dt_max) / h;
+    return std::fmin(kappa_rises ? 2.0 * step : step, 0.5);
 }
 
-// Whether particles end their pushes near a face of the box often (MixedConsts::
-// all_bounds): 2D 64^2, skipping the test over not, steps of 0.1 and less 0.94, 0.3
-// 1.1 to 1.3.
-inline int long_steps(double step, bool kappa_rises) { return step >= (kappa_rises ? 0.05 : 0.2); }
+// Whether particles end their pushes outside the box's cells often (MixedConsts::
+// all_bounds): 2D 64^2, skipping the boundary test inside them over not skipping it,
+// steps of 0.1 and less 0.94, 0.3 1.1 to 1.3.
+inline int long_steps(double step) { return step >= 0.2; }
 
 // Gathering by groups of lanes spares the L1 data pipe, and costs shuffles and
 // weights computed twice (2D) or a turn through shared memory (3D).  It gains
@@ -37,12 +39,11 @@ inline int long_steps(double step, bool kappa_rises) { return step >= (kappa_ris
 // share.  Binned by cell they share them while the particles have moved less than
 // some cells since, and where many particles stand in a cell.  Time of an interval
 // of 200 to 300 pushes by single lanes over that by groups:
-//   2D, one frame: 64^2 to 1024^2 cells, 2 to 128 a cell, step up to 0.3: 0.83 to
-//     0.9; half a cell: 64^2 0.77 to 1.0, 256^2 0.8 (0.1 a cell) to 1.0 (8 a cell),
-//     512^2 0.83 (0.1) to 1.04 (2), 1024^2 1.07 (2), 2048^2 1.2 (0.5); below one a
-//     cell on 1024^2 and 2048^2 at any step 1.0 to 1.27, on 256^2 and 512^2 0.8 to 0.95.
-//     A set that stands together, as one injected at a shock does: 1e5 particles on
-//     512 x 64 cells, half a cell, 1.12.
+//   2D, one frame: 64^2 to 1024^2 cells, 2 to 128 a cell, step up to 0.3: 0.84 to
+//     0.93; half a cell: 64^2 1.04 to 1.1, 256^2 and 512^2 0.85 (0.1 a cell) to 1.02,
+//     1024^2 and 2048^2 1.03 to 1.27, and for sets that stand together, as those
+//     injected at a shock do, 1.1 (3e4 on 512^2, 1e5 on 512 x 64); below one a cell on 1024^2 and 2048^2 at any step 1.0 to 1.27, on 256^2
+//     and 512^2 0.9 to 1.0.
 //   2D, two frames, 8 a cell: step 0.03 0.9, 0.1 0.96, 0.3 0.98 to 1.2, half a cell
 //     1.26 to 1.4; 0.5 a cell: 1.0 to 1.5 at any step.
 //   2D, 100 to 9000 particles, which leave each scheduler a warp that waits for its
@@ -58,7 +59,7 @@ inline bool gathers_in_groups(const GatherLoad &g) {
     if (g.ndim == 2) {
         if (few || 2 * g.n <= (int64_t)g.sm_count * 128) return false;
         if (g.two_frames) return per_cell < 1.0 || g.step >= 0.25;
-        if (g.step >= 0.45) return g.cells >= 4e5 || g.n >= 40000;
+        if (g.step >= 0.45) return true;
         return per_cell < 1.0 && g.cells >= 4e5;
     }
     // a launch that leaves a particle a whole group of lanes (spread_of)

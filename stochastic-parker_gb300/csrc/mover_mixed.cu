@@ -52,8 +52,8 @@ MixedConsts make_mixed_consts(const MoverArgs &a) {
     k.acc_scale[0] = (float)(a.dx / a.cfg_lx);
     k.acc_scale[1] = (float)(a.dy / a.cfg_ly);
     k.acc_scale[2] = (float)(a.dz / a.cfg_lz);
-    k.all_bounds = long_steps(gather_step(a.ndim, a.kpara0, a.dt_max, a.dx, a.dy, a.dz),
-                              a.momentum_dependency != 0);
+    k.all_bounds = long_steps(gather_step(a.ndim, a.kpara0, a.momentum_dependency != 0, a.dt_max,
+                                          a.dx, a.dy, a.dz));
     return k;
 }
 
@@ -218,7 +218,8 @@ MixedRunArgs mixed_run_args(const MoverArgs &a) {
 bool mover_gathers_in_groups(const MoverArgs &a, int64_t n, int sm_count) {
     const double cells = (double)a.nxg * a.nyg * a.nzg;
     return gathers_in_groups({a.ndim, a.time_interp != 0, n, cells, (double)a.n / cells,
-                              gather_step(a.ndim, a.kpara0, a.dt_max, a.dx, a.dy, a.dz), sm_count,
+                              gather_step(a.ndim, a.kpara0, a.momentum_dependency != 0, a.dt_max,
+                                          a.dx, a.dy, a.dz), sm_count,
                               std::fmin(a.dtf / std::fmin(a.dt_min, a.dt_max),
                                         a.chunk_pushes ? (double)a.chunk_pushes : INFINITY)});
 }

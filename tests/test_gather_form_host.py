@@ -14,7 +14,7 @@ CSRC = Path(__file__).resolve().parent.parent / "stochastic-parker_gb300" / "csr
 # launch makes 128 pushes
 POINTS = [
     (2, 0, 64, 8.0, 0.03, 0), (2, 0, 64, 2.0, 0.3, 0), (2, 0, 256, 2.0, 0.01, 0),
-    (2, 0, 256, 0.5, 0.3, 0), (2, 0, 256, 0.1, 0.5, 0), (2, 0, 512, 0.1, 0.5, 0), (2, 0, 64, 2.0, 0.5, 0),
+    (2, 0, 256, 0.5, 0.3, 0), (2, 0, 256, 0.1, 0.5, 0), (2, 0, 64, 2.0, 0.5, 0), (2, 0, 512, 2.0, 0.5, 1),
     (2, 0, 512, 2.0, 0.1, 0), (2, 0, 1024, 2.0, 0.03, 0), (2, 0, 1024, 0.5, 0.3, 1),
     (2, 0, 1024, 2.0, 0.5, 1), (2, 0, 1024, 0.5, 0.5, 1), (2, 0, 2048, 0.1, 0.003, 1),
     (2, 0, 2048, 0.5, 0.5, 1),
@@ -43,17 +43,17 @@ int main() {
         std::printf("%d\n", (int)gathers_in_groups({ndim, two != 0, n, cells, n / cells, step, 152, 128.0}));
     }
     const double nan = std::numeric_limits<double>::quiet_NaN(), d = 1.0 / 128;
-    // kappa ratio 1: half a cell at most; no diffusion: no step; the smallest side
-    std::printf("%.3f %.3f %.3f\n", gather_step(2, 1.0, 1.0, d, d, 1.0),
-                gather_step(3, 0.0, 1.0, d, d, d), gather_step(3, d * d / 8, 0.01, d, 2 * d, d / 2));
+    // half a cell at most; no diffusion: no step; the smallest side, twice at p0
+    std::printf("%.3f %.3f %.3f\n", gather_step(2, 1.0, false, 1.0, d, d, 1.0),
+                gather_step(3, 0.0, true, 1.0, d, d, d),
+                gather_step(3, d * d / 8, true, 0.01, d, 2 * d, d / 2));
     std::printf("%d\n", (int)gathers_in_groups({3, false, 1, 8.0, 0.125, nan, 152, nan}));
     // launches of few pushes, right after a binning: by single lanes, unless each
     // particle has a group of its own
     std::printf("%d %d %d\n", (int)gathers_in_groups({2, true, 2000000, 4e6, 0.5, 0.5, 152, 16.0}),
                 (int)gathers_in_groups({3, true, 1000000, 2e6, 0.5, 0.5, 152, 10.0}),
                 (int)gathers_in_groups({3, true, 30000, 2e6, 0.015, 0.5, 152, 10.0}));
-    std::printf("%d %d %d %d\n", long_steps(0.1, false), long_steps(0.3, false), long_steps(0.1, true),
-                long_steps(0.01, true));
+    std::printf("%d %d %d %d\n", long_steps(0.1), long_steps(0.3), long_steps(0.2), long_steps(0.0));
     return 0;
 }
 """
@@ -72,8 +72,8 @@ def test_forms_at_the_measured_points(tmp_path):
                          check=True).stdout.split("\n")
     got = [int(v) for v in out[:len(POINTS)]]
     assert got == [p[5] for p in POINTS], [p for p, g in zip(POINTS, got) if g != p[5]]
-    # 0.1 = sqrt(2 (d^2 / 8) 0.01) / (d / 2)
-    assert out[len(POINTS)] == "0.500 0.000 0.100"
+    # 0.2 = 2 sqrt(2 (d^2 / 8) 0.01) / (d / 2)
+    assert out[len(POINTS)] == "0.500 0.000 0.200"
     assert out[len(POINTS) + 1] in ("0", "1")
     assert out[len(POINTS) + 2] == "0 0 1"
     assert out[len(POINTS) + 3] == "0 1 1 0"
