@@ -42,8 +42,8 @@ inline int long_steps(double step) { return step >= 0.2; }
 //   2D, one frame: 64^2 to 1024^2 cells, 2 to 128 a cell, step up to 0.3: 0.84 to
 //     0.93; half a cell: 64^2 1.04 to 1.1, 256^2 and 512^2 0.85 (0.1 a cell) to 1.02,
 //     1024^2 and 2048^2 1.03 to 1.27, and for sets that stand together, as those
-//     injected at a shock do, 1.1 (3e4 on 512^2, 1e5 on 512 x 64); below one a cell on 1024^2 and 2048^2 at any step 1.0 to 1.27, on 256^2
-//     and 512^2 0.9 to 1.0.
+//     injected at a shock do, 1.1 (3e4 on 512^2, 1e5 on 512 x 64); below one a cell on
+//     1024^2 and 2048^2 at any step 1.0 to 1.27, on 256^2 and 512^2 0.9 to 1.0.
 //   2D, two frames, 8 a cell: step 0.03 0.9, 0.1 0.96, 0.3 0.98 to 1.2, half a cell
 //     1.26 to 1.4; 0.5 a cell: 1.0 to 1.5 at any step.
 //   2D, 100 to 9000 particles, which leave each scheduler a warp that waits for its

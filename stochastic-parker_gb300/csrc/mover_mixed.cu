@@ -72,8 +72,9 @@ __device__ __forceinline__ int64_t spread_index(int spread, int64_t n, bool &val
 // which leaves one round of loads of the group's four; from there, and in 2D, the
 // lanes of a warp only keep one another waiting, which is worth more warps while
 // each scheduler has at most one.  Intervals of 300, 2000, 10 000 and 40 000
-// particles with 1 -> these lanes each: 3D, two frames 2.33 -> 0.77, 2.43 -> 0.83,
-// 2.45 -> 1.16 and 2.82 -> 2.12 ms; 2D 0.78 -> 0.63, 0.80 -> 0.68 and no change.
+// particles with 1 -> these lanes each, gathering by groups: 3D, two frames 2.33 ->
+// 0.77, 2.43 -> 0.83, 2.45 -> 1.16 and 2.82 -> 2.12 ms; 2D 0.78 -> 0.63, 0.80 -> 0.68
+// and no change (2D launches of that size now gather by single lanes, 0.75 of that).
 // Past these lines: 2D, 40 000 particles, 2 lanes 0.88 -> 1.08 ms; 3D, 2000 particles,
 // 32 lanes 0.83 -> 0.99 ms.
 int spread_of(int ndim, int64_t n, int sm_count) {
