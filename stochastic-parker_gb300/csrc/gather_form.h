@@ -18,14 +18,14 @@ struct GatherLoad {
     double pushes;     // of a particle in the launch, at most
 };
 
-// Half a cell is what the step's diffusion limit allows.  Where kappa rises with p,
-// as p^(4/3) or so, twice what it is at p0: particles of sqrt(10) p0.
+// Above half a cell the step's diffusion limit shortens it to that.  Where kappa rises
+// with p, as p^(4/3) or so, twice what it is at p0: particles of sqrt(10) p0.
 inline double gather_step(int ndim, double kpara0, bool kappa_rises, double dt_max, double dx,
                           double dy, double dz) {
     double h = std::fmin(dx, dy);
     if (ndim == 3) h = std::fmin(h, dz);
     const double step = std::sqrt(2.0 * std::fabs(kpara0) * dt_max) / h;
-    return std::fmin(kappa_rises ? 2.0 * step : step, 0.5);
+    return kappa_rises ? 2.0 * step : step;
 }
 
 // Whether particles end their pushes outside the box's cells often (MixedConsts::
@@ -47,7 +47,9 @@ inline int long_steps(double step) { return step >= 0.2; }
 //   2D, two frames, 8 a cell: step 0.03 0.9, 0.1 0.96, 0.3 0.98 to 1.2, half a cell
 //     1.26 to 1.4; 0.5 a cell: 1.0 to 1.5 at any step.
 //   2D, 100 to 9000 particles, which leave each scheduler a warp that waits for its
-//     own chain of operations: 0.75 to 0.83 (one frame), 0.74 to 0.9 (two).
+//     own chain of operations: 0.75 to 0.83 (one frame), 0.74 to 0.9 (two); where dt_max
+//     is far above the diffusion limit (steps of 2 cells and more by it), from 2500
+//     particles on 1.08 to 1.2.
 //   3D, one frame: step 0.03, 0.5 to 32 a cell: 0.78 to 0.98; step 0.1, 0.5 and 2 a
 //     cell: 0.9 to 1.01, 8 and 32: 1.11 to 1.17; step 0.3: 1.0 to 1.07; half a cell
 //     1.1 to 1.3; 0.1 a cell: 0.92 to 1.17.
@@ -57,7 +59,9 @@ inline bool gathers_in_groups(const GatherLoad &g) {
     const double per_cell = g.per_cell;
     const bool few = g.pushes <= 16.0;
     if (g.ndim == 2) {
-        if (few || 2 * g.n <= (int64_t)g.sm_count * 128) return false;
+        if (few) return false;
+        if (2 * g.n <= (int64_t)g.sm_count * 128)
+            return g.step >= 2.0 && 8 * g.n > (int64_t)g.sm_count * 128;
         if (g.two_frames) return per_cell < 1.0 || g.step >= 0.25;
         if (g.step >= 0.45) return true;
         return per_cell < 1.0 && g.cells >= 4e5;

@@ -15,6 +15,7 @@ CSRC = Path(__file__).resolve().parent.parent / "stochastic-parker_gb300" / "csr
 POINTS = [
     (2, 0, 64, 8.0, 0.03, 0), (2, 0, 64, 2.0, 0.3, 0), (2, 0, 256, 2.0, 0.01, 0),
     (2, 0, 256, 0.5, 0.3, 0), (2, 0, 256, 0.1, 0.5, 0), (2, 0, 64, 2.0, 0.5, 0), (2, 0, 512, 2.0, 0.5, 1),
+    (2, 0, 64, 2.0, 3.0, 1), (2, 1, 64, 0.4, 3.0, 0), (2, 1, 1024, 0.006, 2.9, 1),
     (2, 0, 512, 2.0, 0.1, 0), (2, 0, 1024, 2.0, 0.03, 0), (2, 0, 1024, 0.5, 0.3, 1),
     (2, 0, 1024, 2.0, 0.5, 1), (2, 0, 1024, 0.5, 0.5, 1), (2, 0, 2048, 0.1, 0.003, 1),
     (2, 0, 2048, 0.5, 0.5, 1),
@@ -43,7 +44,7 @@ int main() {
         std::printf("%d\n", (int)gathers_in_groups({ndim, two != 0, n, cells, n / cells, step, 152, 128.0}));
     }
     const double nan = std::numeric_limits<double>::quiet_NaN(), d = 1.0 / 128;
-    // half a cell at most; no diffusion: no step; the smallest side, twice at p0
+    // sqrt(2) / d; no diffusion: no step; the smallest side, twice at p0
     std::printf("%.3f %.3f %.3f\n", gather_step(2, 1.0, false, 1.0, d, d, 1.0),
                 gather_step(3, 0.0, true, 1.0, d, d, d),
                 gather_step(3, d * d / 8, true, 0.01, d, 2 * d, d / 2));
@@ -73,7 +74,7 @@ def test_forms_at_the_measured_points(tmp_path):
     got = [int(v) for v in out[:len(POINTS)]]
     assert got == [p[5] for p in POINTS], [p for p, g in zip(POINTS, got) if g != p[5]]
     # 0.2 = 2 sqrt(2 (d^2 / 8) 0.01) / (d / 2)
-    assert out[len(POINTS)] == "0.500 0.000 0.200"
+    assert out[len(POINTS)] == "181.019 0.000 0.200"
     assert out[len(POINTS) + 1] in ("0", "1")
     assert out[len(POINTS) + 2] == "0 0 1"
     assert out[len(POINTS) + 3] == "0 1 1 0"

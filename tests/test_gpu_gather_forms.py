@@ -52,6 +52,7 @@ def _moved(eng, start, idx, **kw):
 @pytest.mark.parametrize("ndim,two,step,n,total,parts", [
     (2, False, 0.5, 36, 40000, (9000, 3000, 300, 33, 1)),   # groups -> lanes
     (2, True, 0.1, 128, 40000, (12000, 3000, 1)),           # lanes -> groups -> lanes
+    (2, True, 3.0, 100, 20000, (9000, 3000, 2000, 1)),      # groups -> lanes at 2000
     (3, False, 0.05, 20, 60000, (20000, 3000, 1)),          # lanes -> groups
     (3, True, 0.01, 20, 60000, (20000, 3000, 1)),
 ])
